@@ -195,11 +195,10 @@ struct StreamFree {
 };
 
 static int finish_index(Index& ix, cudaStream_t st) {
-  float init[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  B2K_CUDA(cudaMemcpyAsync(ix.stats_dev, init, sizeof(init), cudaMemcpyHostToDevice, st));
+  B2K_CUDA(cudaMemsetAsync(ix.stats_dev, 0, kStatsLen * sizeof(float), st));
   launch_prep_index(&ix, st);
   B2K_CUDA(cudaGetLastError());
-  float stats[8];
+  float stats[kStatsLen];
   B2K_CUDA(cudaMemcpyAsync(stats, ix.stats_dev, sizeof(stats), cudaMemcpyDeviceToHost, st));
   B2K_CUDA(cudaStreamSynchronize(st));
   ix.xn_max = stats[0];
@@ -286,6 +285,14 @@ static int ensure_row_groups(Index& ix) {
   return make_row_groups(ix);
 }
 
+static OperandStats bf16_stats(const float* stats) {
+  OperandStats s;
+  s.xh = stats[3];
+  s.ex = stats[4];
+  for (int i = 0; i < 3; ++i) s.part[i] = stats[8 + i];
+  return s;
+}
+
 static int ensure_bf16(Index& ix) {
   std::lock_guard<std::mutex> lock(ix.mu);
   if (ix.bf16_ready) return B2K_OK;
@@ -297,11 +304,10 @@ static int ensure_bf16(Index& ix) {
   B2K_CUDA(cudaMalloc(&ix.Xh, (size_t)ix.n_pad_tc * ix.dp * sizeof(uint16_t)));
   launch_prep_index_bf16(&ix, ix.Xh, st, ix.xperm);
   B2K_CUDA(cudaGetLastError());
-  float stats[8];
+  float stats[kStatsLen];
   B2K_CUDA(cudaMemcpyAsync(stats, ix.stats_dev, sizeof(stats), cudaMemcpyDeviceToHost, st));
   B2K_CUDA(cudaStreamSynchronize(st));
-  ix.xh_max = stats[3];
-  ix.ex_max = stats[4];
+  ix.hs = bf16_stats(stats);
   if (!tensor_map_2d_bf16(&ix.tmap_b, ix.Xh, (uint64_t)ix.dp, (uint64_t)ix.n_pad_tc, kTcBK, kTcBN))
     return fail(B2K_ECUDA, "cuTensorMapEncodeTiled failed for the reference rows");
   // norm columns of the reference rows and the matching query-side ones
@@ -334,7 +340,7 @@ static int ensure_tf32(Index& ix) {
   B2K_CUDA(cudaMalloc(&ix.taug_ones, (size_t)kTcBM * kTcAugF * sizeof(float)));
   launch_prep_aug_tf32(&ix, ix.Xtaug, ix.taug_ones, st, ix.xperm);
   B2K_CUDA(cudaGetLastError());
-  float stats[8];
+  float stats[kStatsLen];
   B2K_CUDA(cudaMemcpyAsync(stats, ix.stats_dev, sizeof(stats), cudaMemcpyDeviceToHost, st));
   B2K_CUDA(cudaStreamSynchronize(st));
   ix.xt_max = stats[6];
@@ -577,7 +583,7 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
   if (u8) mode = B2K_MODE_U8;
   if (mode == B2K_MODE_AUTO)
     mode = (!ix.range_ok || k > kMaxK) ? B2K_MODE_EXACT
-           : (ix.d >= 16 && ix.n >= 2048) ? B2K_MODE_BF16
+           : (ix.d >= kTcMinD && ix.n >= kTcMinN) ? B2K_MODE_BF16
                                          : B2K_MODE_FP32;
   if (mode != B2K_MODE_EXACT && !u8 && (!ix.range_ok || k > kMaxK)) mode = B2K_MODE_EXACT;
   if (stats) {
@@ -872,17 +878,16 @@ int knn_device_run(Index& ix, const float* dQ, int64_t m, int k, int exclude_sel
 }
 int injected_fault() { return fault_mode(); }
 int index_prepare_bf16_stats(Index& ix, uint16_t* Xh, uint16_t* Xaug, uint16_t* ones,
-                             cudaStream_t st, float* xh_max, float* ex_max) {
+                             cudaStream_t st, OperandStats* out) {
   std::lock_guard<std::mutex> lock(ix.mu);
   launch_prep_index_bf16(&ix, Xh, st);
   B2K_CUDA(cudaGetLastError());
   launch_prep_aug(&ix, Xaug, ones, st);
   B2K_CUDA(cudaGetLastError());
-  float stats[8];
+  float stats[kStatsLen];
   B2K_CUDA(cudaMemcpyAsync(stats, ix.stats_dev, sizeof(stats), cudaMemcpyDeviceToHost, st));
   B2K_CUDA(cudaStreamSynchronize(st));
-  *xh_max = stats[3];
-  *ex_max = stats[4];
+  *out = bf16_stats(stats);
   return B2K_OK;
 }
 
@@ -948,7 +953,7 @@ static int build_from_device(b2k_index* h, const float* src, cudaMemcpyKind kind
   B2K_CUDA(cudaMalloc(&ix.center, (size_t)ix.d * sizeof(float)));
   B2K_CUDA(cudaMalloc(&ix.colsum, (size_t)ix.d * sizeof(double)));
   B2K_CUDA(cudaMalloc(&ix.nx64, (size_t)ix.n * sizeof(double)));
-  B2K_CUDA(cudaMalloc(&ix.stats_dev, 8 * sizeof(float)));
+  B2K_CUDA(cudaMalloc(&ix.stats_dev, kStatsLen * sizeof(float)));
   if (kind == cudaMemcpyDeviceToDevice && user_st) {
     B2K_CUDA(cudaMemcpyAsync(ix.X, src, bytes, kind, user_st));
     B2K_CUDA(cudaStreamSynchronize(user_st));
@@ -1144,7 +1149,7 @@ static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int ex
                         bool counted = false, bool sort_rows = true) {
   StreamFree fr{st, {}};
   int rc;
-  int mode = (!admit_all && ix.d >= 16 && ix.n >= 2048) ? B2K_MODE_BF16 : B2K_MODE_FP32;
+  int mode = (!admit_all && ix.d >= kTcMinD && ix.n >= kTcMinN) ? B2K_MODE_BF16 : B2K_MODE_FP32;
   if (mode == B2K_MODE_BF16 && (rc = ensure_bf16(ix))) return rc;
   const bool tc = mode == B2K_MODE_BF16;
   const int64_t bm = tc ? kTcBM : kSimtBM;

@@ -124,7 +124,7 @@ struct BProb {
   int dp = 0, KB = 0, n_tiles = 0, m_pad = 0, m_tiles = 0, kmax = 0;
   int dpg = -1;         // dp group
   int64_t a_row0 = 0, b_row0 = 0, pad0 = 0, row0 = 0;
-  float xh_max = 0, ex_max = 0;
+  OperandStats xs;
   // tuned layout
   int ew = 8, halves = 2, S = 1, tps = 0, S_lists = 2, cap = kListCap;
   int launch = -1, group = -1;
@@ -254,22 +254,21 @@ int build_fixed(b2k_batch* b, cudaStream_t st) {
     return bfail(B2K_ECUDA, "cuTensorMapEncodeTiled failed for the norm columns");
   // reference operands, once per distinct index
   bool ones_done = false;
-  std::map<const Index*, std::pair<float, float>> stats;
+  std::map<const Index*, OperandStats> stats;
   for (auto& p : b->probs) {
     if (!p.in_graph) continue;
     auto s = stats.find(p.ix);
     if (s == stats.end()) {
       DpGroup& g = b->dpg[p.dpg];
-      float xh = 0, ex = 0;
+      OperandStats os;
       rc = index_prepare_bf16_stats(*p.ix, g.B + (size_t)p.b_row0 * g.dp,
                                     g.Baug + (size_t)p.b_row0 * kTcAug,
-                                    ones_done ? nullptr : b->ones, st, &xh, &ex);
+                                    ones_done ? nullptr : b->ones, st, &os);
       if (rc) return rc;
       ones_done = true;
-      s = stats.emplace(p.ix, std::make_pair(xh, ex)).first;
+      s = stats.emplace(p.ix, os).first;
     }
-    p.xh_max = s->second.first;
-    p.ex_max = s->second.second;
+    p.xs = s->second;
   }
   const int P = b->n_graph;
   if ((rc = o.alloc(&b->zero_block, 8 + (size_t)P))) return rc;
@@ -301,10 +300,10 @@ int build_fixed(b2k_batch* b, cudaStream_t st) {
     q.d = p.ix->d;
     q.dp = p.dp;
     q.mode = B2K_MODE_BF16;
+    q.parts = operand_parts(p.ix->d);
     q.center = p.ix->center;
-    q.xh_max = p.xh_max;
+    q.xs = p.xs;
     q.nx_max = p.ix->nx_max;
-    q.ex_max = p.ex_max;
     q.E = b->E + p.pad0;
     q.Ah = g.A + (size_t)p.a_row0 * g.dp;
     q.nq = b->nq + p.pad0;

@@ -19,6 +19,28 @@ constexpr int kTcAugF = 8;   // tf32 norm columns (one K=8 step, 32 bytes like k
 constexpr int kTcBKu = 128;  // u8 elements per 128-byte swizzle row
 constexpr int kU8MaxK = 16;  // largest k of the exact u8 screen
 constexpr int kU8MaxD = 16384;  // ||x||^2 and -2<q, x> of u8 rows fit int32
+// Narrow rows leave most of a 64-column operand block empty, and the block
+// costs the same full or not (the epilogue bounds a 128 x 256 tile: multiplying
+// only the used columns was measured and was 2 to 4% slower).  So rows of at
+// most 21 features are split into bf16 parts (hi + mid, up to 10 features
+// hi + mid + lo) whose cross products fill the block: <q, x> then carries 16 or
+// 24 bits instead of 8, and the certified band shrinks with it.  With whole
+// bf16 operands the band of an 8-feature row (about 0.1 against a k-th squared
+// distance of 0.3 on 200,000 N(0, 1) rows) would hold most of a query's lists.
+__host__ __device__ constexpr int operand_parts(int d) { return d <= 10 ? 3 : d <= 21 ? 2 : 1; }
+// operand columns in use: parts 2 = (h,h)(h,m)(m,h), parts 3 adds
+// (m,m)(h,l)(l,h), written (query part, row part)
+__host__ __device__ constexpr int operand_cols(int d) {
+  return operand_parts(d) == 3 ? 6 * d : operand_parts(d) == 2 ? 3 * d : d;
+}
+// Narrowest rows AUTO and the radius search send to the tensor cores.  200,003
+// x 8 rows, 50,021 queries, k = 5: the call takes 2.60 ms (screen 2.05 ms), on
+// the CUDA cores 17.54 ms (screen 17.03 ms).  Rows of one or two features stay
+// there: at 10^6 rows a plane holds more rows inside the accumulation error
+// (16 ulp of ||x||^2 an addition) than the lists take.
+constexpr int kTcMinD = 3;
+constexpr int64_t kTcMinN = 2048;
+constexpr int kStatsLen = 12;  // floats of Index::stats_dev (prep.cu)
 constexpr int kSimtBM = 128; // query rows per CUDA-core tile
 constexpr int kSimtBN = 64;  // reference rows per CUDA-core tile
 constexpr int kListCap = 512;      // screen list entries per (split, query)
@@ -39,6 +61,13 @@ struct ScreenOut {
   int m_pad;
 };
 
+// Maxima over the rows of a screen operand x^ (the sum of its parts).
+struct OperandStats {
+  float xh = 0;      // ||x^||
+  float ex = 0;      // ||(x - center) - x^||
+  float part[3] = {0, 0, 0};  // ||hi||, ||mid||, ||lo|| (one part: ||x^||, 0, 0)
+};
+
 // Device-resident index (one per fitted estimator).
 struct Index {
   int device = 0;
@@ -50,7 +79,7 @@ struct Index {
   float* nx32 = nullptr;     // [n] fl32(||x - center||^2)
   double* nx64 = nullptr;    // [n] ||x - center||^2 in float64
   // screen statistics (device scalars, then cached on host)
-  float* stats_dev = nullptr;  // [8]: see prep kernels
+  float* stats_dev = nullptr;  // [kStatsLen]: see prep kernels
   float xn_max = 0, nx_max = 0;  // max ||fp32 operand||, max ||x - center||^2
   float ex32_max = 0;            // max ||(x - center) - fp32 operand||
   bool range_ok = false;         // all |x| in {0} U [2^-60, 2^50]
@@ -59,7 +88,7 @@ struct Index {
   int64_t n_pad_tc = 0;          // multiple of kTcBN
   int32_t dp = 0;                // d padded to a multiple of kTcBK
   uint16_t* Xh = nullptr;        // [n_pad_tc, dp]
-  float xh_max = 0, ex_max = 0;  // max ||bf16 operand||, max ||(x - center) - bf16 operand||
+  OperandStats hs;               // of the bf16 operand
   CUtensorMap tmap_b;            // TMA map over Xh, box 64 x 256
   uint16_t* Xaug = nullptr;      // [n_pad_tc, 16] bf16 [n_hi, n_mid, n_lo, 0...] of ||x - c||^2
   uint16_t* aug_ones = nullptr;  // [128, 16] bf16 [1, 1, 1, 0...] (query side)
@@ -145,8 +174,10 @@ struct PrepProblem {
   const float* Q;
   int64_t m, m_pad;
   int d, dp, mode;
+  int parts;                     // bf16 parts of an operand value (1 in the other modes)
   const float* center;
-  float xh_max, nx_max, ex_max;  // operand statistics of the index for `mode`
+  OperandStats xs;               // operand statistics of the index for `mode`
+  float nx_max;
   float* E;
   uint16_t* Ah;                  // [m_pad, dp] (bf16 mode)
   float* At;                     // [m_pad, dp] (tf32 mode; dp is then the tf32 width)
@@ -370,7 +401,7 @@ int injected_fault();  // B2K_FAULT: 0 none, 1 alloc, 2 launch, 3 timeout
 // bf16 operand rows and norm columns of an index into caller buffers, and the
 // operand statistics the query bound needs (synchronises st)
 int index_prepare_bf16_stats(Index& ix, uint16_t* Xh, uint16_t* Xaug, uint16_t* ones,
-                             cudaStream_t st, float* xh_max, float* ex_max);
+                             cudaStream_t st, OperandStats* stats);
 bool tensor_map_2d_bf16(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer,
                         uint32_t box_inner, uint32_t box_outer, int swizzle_bytes = 128);
 bool tensor_map_2d_f32(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer,

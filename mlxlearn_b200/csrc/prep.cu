@@ -20,7 +20,12 @@
 //     + 2^-50 ||y_q||^2,  times (1 + 2^-16), plus dp 2^-120 for underflow,
 // with the x-side norms replaced by their maxima over the index and
 //   g = (d + 4) u (1.01)          fp32 FMA chains (CUDA-core screen),
-//   g = (dp + 16) 2^-20           tcgen05 fp32 accumulation (16 ulp per add).
+//   g = (dp + 32) 2^-20           tcgen05 fp32 accumulation (16 ulp per add).
+// Rows of at most 21 features are split into bf16 parts (operand_parts): with
+// q^ = sum of a_i, x^ = sum of b_j, the screen sums the products listed at
+// operand_cols and drops the others, which adds their bound 2 sum |a_i||b_j|
+// to E; the accumulation term takes the sum of |a_i||b_j| over the kept
+// products in the place of |q^||x^|.
 // The tf32 screen (kind::tf32) works the same way on operands rounded to
 // tf32 here (10 explicit mantissa bits, so the tensor core reads them
 // exactly) with the norm split into three tf32 parts in 8 columns; its
@@ -75,7 +80,8 @@ __global__ void center_kernel(const double* __restrict__ sums, int64_t n, int d,
 
 // stats: [0] max |x^| fp32 operand, [1] max ||y||^2, [2] range violations (int),
 //        [3] max |x~| bf16 operand, [4] max |e| bf16, [5] max |e| fp32,
-//        [6] max |x~| tf32 operand, [7] max |e| tf32
+//        [6] max |x~| tf32 operand, [7] max |e| tf32,
+//        [8] [9] [10] max |part| of the bf16 operand's parts
 __global__ void prep_index_kernel(const float* __restrict__ X, int64_t n, int d,
                                   const float* __restrict__ center, float* __restrict__ nx32,
                                   double* __restrict__ nx64, float* __restrict__ stats) {
@@ -109,6 +115,35 @@ __global__ void prep_index_kernel(const float* __restrict__ X, int64_t n, int d,
   }
 }
 
+// The bf16 parts of a centred fp32 value (the differences are exact in fp32).
+__device__ __forceinline__ void bf16_split(float v, int parts, float (&p)[3]) {
+  p[0] = __bfloat162float(__float2bfloat16_rn(v));
+  p[1] = p[2] = 0.0f;
+  if (parts > 1) {
+    const float r = v - p[0];
+    p[1] = __bfloat162float(__float2bfloat16_rn(r));
+    if (parts > 2) p[2] = __bfloat162float(__float2bfloat16_rn(r - p[1]));
+  }
+}
+
+// Feature f of an operand row, its parts in the column blocks of operand_cols
+// (`scale` 1 on the row side, -2 on the query side: exact).
+template <bool QUERY>
+__device__ __forceinline__ void store_parts(__nv_bfloat16* row, int d, int f, int parts,
+                                            const float (&p)[3]) {
+  constexpr float scale = QUERY ? -2.0f : 1.0f;
+  row[f] = __float2bfloat16_rn(scale * p[0]);
+  if (parts > 1) {
+    row[d + f] = __float2bfloat16_rn(scale * p[QUERY ? 0 : 1]);
+    row[2 * d + f] = __float2bfloat16_rn(scale * p[QUERY ? 1 : 0]);
+  }
+  if (parts > 2) {
+    row[3 * d + f] = __float2bfloat16_rn(scale * p[1]);
+    row[4 * d + f] = __float2bfloat16_rn(scale * p[QUERY ? 0 : 2]);
+    row[5 * d + f] = __float2bfloat16_rn(scale * p[QUERY ? 2 : 0]);
+  }
+}
+
 __global__ void prep_index_bf16_kernel(const float* __restrict__ X, int64_t n, int d,
                                        int64_t n_pad, int dp, const float* __restrict__ center,
                                        const int* __restrict__ rows,
@@ -118,31 +153,45 @@ __global__ void prep_index_bf16_kernel(const float* __restrict__ X, int64_t n, i
   int lane = threadIdx.x & 31;
   if (row >= n_pad) return;
   __nv_bfloat16* xh = Xh + row * dp;
-  if (row >= n) {
-    // padding rows: zero operands (their NaN norm column keeps them out)
-    for (int i = lane; i < dp; i += 32) xh[i] = __float2bfloat16_rn(0.0f);
-    return;
-  }
+  const int parts = operand_parts(d);
+  const int cols = row < n ? operand_cols(d) : 0;
+  // padding columns, and padding rows whole (their NaN norm column keeps them out)
+  for (int i = cols + lane; i < dp; i += 32) xh[i] = __float2bfloat16_rn(0.0f);
+  if (row >= n) return;
   const float* x = X + (rows ? (int64_t)rows[row] : row) * d;
-  double hn = 0.0, en = 0.0, yy = 0.0;
-  for (int i = lane; i < dp; i += 32) {
-    const float v = i < d ? x[i] : 0.0f;
-    const float c = i < d ? center[i] : 0.0f;
+  double hn = 0.0, en = 0.0, yy = 0.0, pn[3] = {0.0, 0.0, 0.0};
+  for (int i = lane; i < d; i += 32) {
+    const float v = x[i], c = center[i];
     const double y = (double)v - (double)c;
-    const __nv_bfloat16 h = __float2bfloat16_rn(v - c);
-    xh[i] = h;
-    const double hv = (double)__bfloat162float(h);
+    float p[3];
+    bf16_split(v - c, parts, p);
+    store_parts<false>(xh, d, i, parts, p);
+    const double hv = ((double)p[0] + (double)p[1]) + (double)p[2];
     const double e = y - hv;
     hn += hv * hv;
     en += e * e;
     yy += y * y;
+#pragma unroll
+    for (int t = 0; t < 3; ++t) pn[t] += (double)p[t] * (double)p[t];
   }
   hn = warp_sum(hn);
   en = warp_sum(en);
   yy = warp_sum(yy);
+  if (parts > 1) {
+#pragma unroll
+    for (int t = 0; t < 3; ++t) pn[t] = warp_sum(pn[t]);
+  }
   if (lane == 0) {
-    atomic_max_pos(stats + 3, __double2float_ru(sqrt(hn) * (1.0 + 1e-15)));
+    const float h = __double2float_ru(sqrt(hn) * (1.0 + 1e-15));
+    atomic_max_pos(stats + 3, h);
     atomic_max_pos(stats + 4, __double2float_ru(sqrt(en) * (1.0 + 1e-15) + 0x1p-50 * sqrt(yy)));
+    if (parts == 1) {
+      atomic_max_pos(stats + 8, h);
+    } else {
+#pragma unroll
+      for (int t = 0; t < 3; ++t)
+        atomic_max_pos(stats + 8 + t, __double2float_ru(sqrt(pn[t]) * (1.0 + 1e-15)));
+    }
   }
 }
 
@@ -242,7 +291,9 @@ __global__ void prep_aug_kernel(const double* __restrict__ nx64, int64_t n, int6
 }
 
 // One query row: error bound E, the bf16 operand row (bf16 mode), ||y||^2.
-__device__ __forceinline__ void prep_query_row(const PrepProblem& P, int64_t row, int lane) {
+// SPLIT: more than one bf16 part (operand_parts).
+template <bool SPLIT>
+__device__ __forceinline__ void prep_query_row_as(const PrepProblem& P, int64_t row, int lane) {
   const double u = 0x1p-24;
   const bool bf16 = P.mode == B2K_MODE_BF16;
   const bool tf32 = P.mode == B2K_MODE_TF32;
@@ -258,9 +309,14 @@ __device__ __forceinline__ void prep_query_row(const PrepProblem& P, int64_t row
     return;
   }
   const float* q = P.Q + row * d;
-  double yy = 0.0, hn = 0.0, en = 0.0;
+  const int parts = SPLIT ? P.parts : 1;
+  double yy = 0.0, hn = 0.0, en = 0.0, pn[3] = {0.0, 0.0, 0.0};
   bool ok = true;
-  const int width = tc ? dp : d;
+  if (SPLIT)
+    for (int i = operand_cols(d) + lane; i < dp; i += 32)
+      Ah[row * dp + i] = __float2bfloat16_rn(0.0f);
+  // one part: the loop writes the padding columns too
+  const int width = tc && !SPLIT ? dp : d;
   for (int i = lane; i < width; i += 32) {
     const float v = i < d ? q[i] : 0.0f;
     const float c = i < d ? P.center[i] : 0.0f;
@@ -269,9 +325,15 @@ __device__ __forceinline__ void prep_query_row(const PrepProblem& P, int64_t row
     const float h32 = v - c;
     double hv;
     if (bf16) {
-      const __nv_bfloat16 h = __float2bfloat16_rn(h32);
-      hv = (double)__bfloat162float(h);
-      Ah[row * dp + i] = __float2bfloat16_rn(-2.0f * __bfloat162float(h));  // exact
+      float p[3];
+      bf16_split(h32, parts, p);
+      store_parts<true>(Ah + row * dp, d, i, parts, p);
+      hv = (double)p[0];
+      if (SPLIT) {
+        hv += (double)p[1] + (double)p[2];
+#pragma unroll
+        for (int t = 0; t < 3; ++t) pn[t] += (double)p[t] * (double)p[t];
+      }
     } else if (tf32) {
       const float h = tf32_rne(h32);
       hv = (double)h;
@@ -287,23 +349,47 @@ __device__ __forceinline__ void prep_query_row(const PrepProblem& P, int64_t row
   yy = warp_sum(yy);
   hn = warp_sum(hn);
   en = warp_sum(en);
+  if (parts > 1) {
+#pragma unroll
+    for (int t = 0; t < 3; ++t) pn[t] = warp_sum(pn[t]);
+  }
   ok = __all_sync(0xffffffffu, ok);
   if (lane == 0) {
     const double qh = sqrt(hn) * (1.0 + 1e-15);
     const double eq = sqrt(en) * (1.0 + 1e-15) + 0x1p-50 * sqrt(yy);
-    const double XH = P.xh_max, EX = P.ex_max, NX = P.nx_max;
+    const double XH = P.xs.xh, EX = P.xs.ex, NX = P.nx_max;
+    // kept and dropped products of the parts (one part: |q^||x^| and nothing)
+    double kept = qh * XH, dropped = 0.0;
+    if (parts > 1) {
+      const double a0 = sqrt(pn[0]) * (1.0 + 1e-15), a1 = sqrt(pn[1]) * (1.0 + 1e-15);
+      const double b0 = P.xs.part[0], b1 = P.xs.part[1];
+      kept = a0 * b0 + a0 * b1 + a1 * b0;
+      dropped = a1 * b1;
+      if (parts > 2) {
+        const double a2 = sqrt(pn[2]) * (1.0 + 1e-15), b2 = P.xs.part[2];
+        kept += a1 * b1 + a0 * b2 + a2 * b0;
+        dropped = a1 * b2 + a2 * b1 + a2 * b2;
+      }
+    }
     // tensor cores: dp feature columns + 16 norm columns accumulated in fp32;
     // the accumulation also carries ||y_x||^2 itself (the g * NX term)
     const double g = bf16   ? (double)(dp + kTcAug + 16) * 0x1p-20
                      : tf32 ? (double)(dp + kTcAugF + 16) * 0x1p-20
                             : (double)(d + 4) * u * 1.01;
-    double bound = 2.0 * (qh * EX + eq * XH + eq * EX) + 2.0 * g * qh * XH + 2.0 * u * NX +
-                   2.0 * u * qh * XH * 1.01 + 0x1p-50 * yy + (tc ? g * NX * 1.01 : 0.0);
-    bound = bound * (1.0 + 0x1p-16) + (double)width * 0x1p-120;
+    double bound = 2.0 * (qh * EX + eq * XH + eq * EX + dropped) + 2.0 * g * kept + 2.0 * u * NX +
+                   2.0 * u * kept * 1.01 + 0x1p-50 * yy + (tc ? g * NX * 1.01 : 0.0);
+    bound = bound * (1.0 + 0x1p-16) + (double)(tc ? dp : d) * 0x1p-120;
     P.E[row] = __double2float_ru(bound);
     if (P.nq) P.nq[row] = yy;
     if (!ok) atomicOr(P.flags, 1);
   }
+}
+
+__device__ __forceinline__ void prep_query_row(const PrepProblem& P, int64_t row, int lane) {
+  if (P.parts > 1)
+    prep_query_row_as<true>(P, row, lane);
+  else
+    prep_query_row_as<false>(P, row, lane);
 }
 
 __global__ void prep_queries_kernel(const __grid_constant__ PrepProblem P) {
@@ -416,9 +502,14 @@ PrepProblem prep_problem(const Index* ix, const float* Q, int64_t m, int64_t m_p
   P.dp = tf32 ? (ix->d + kTcBKf - 1) / kTcBKf * kTcBKf : (ix->d + kTcBK - 1) / kTcBK * kTcBK;
   P.mode = mode;
   P.center = ix->center;
-  P.xh_max = bf16 ? ix->xh_max : tf32 ? ix->xt_max : ix->xn_max;
+  P.parts = bf16 ? operand_parts(ix->d) : 1;
   P.nx_max = ix->nx_max;
-  P.ex_max = bf16 ? ix->ex_max : tf32 ? ix->ext_max : ix->ex32_max;
+  if (bf16) {
+    P.xs = ix->hs;
+  } else {
+    P.xs.xh = tf32 ? ix->xt_max : ix->xn_max;
+    P.xs.ex = tf32 ? ix->ext_max : ix->ex32_max;
+  }
   P.E = qp.E;
   P.Ah = qp.Ah;
   P.At = qp.At;

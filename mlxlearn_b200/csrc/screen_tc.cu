@@ -45,7 +45,7 @@
 // per (split, column group, row).
 //
 // Operands are the centred coordinates rounded to bf16 (A = -2 bf16(q - c),
-// B = bf16(x - c)); the certified error bound of v is derived in prep.cu with
+// B = bf16(x - c); narrow rows in bf16 parts, operand_parts); the certified error bound of v is derived in prep.cu with
 // g = (dp + 32) 2^-20 for the tensor-core fp32 accumulation.
 //
 // The TF32 instantiation is the plain (full-width) form on the tensor cores:

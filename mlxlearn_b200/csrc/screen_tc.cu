@@ -15,18 +15,22 @@
 //               work unit; reference tiles B (256 rows x 64 columns, 128-byte
 //               swizzle) into an NST-deep shared-memory ring, the norm
 //               columns (256 rows x 16, 32-byte swizzle) with the last block.
-//   warp 1      MMA issuer: tcgen05.mma kind::f16, M=128 N=256 K=16, fp32
-//               accumulators in TMEM, double-buffered (2 x 256 columns).
-//               It polls one mbarrier (go) per chunk of C = min(KB, stages/2)
-//               64-column blocks, i.e. once per tile for d <= 128: the thread
-//               issuing MMAs runs only about one MMA ahead of the tensor pipe,
-//               so every poll it makes idles the pipe; a poll per block plus
-//               one for the accumulator cost up to 2x in measured MMA
-//               throughput.
-//   last warp   gate: per chunk, waits for its TMA stages (at a tile's first
-//               chunk also for the epilogue's release of the accumulator
-//               buffer; at a unit's start for the query tile), then arrives
-//               on go.  A chunk never needs more stages than the ring holds.
+//   warp 1 and  MMA issuers: tcgen05.mma kind::f16, M=128 N=256 K=16, fp32
+//   last warp   accumulators in TMEM, double-buffered (2 x 256 columns).  When
+//               the ring holds two tiles the issuers take turns, one per
+//               accumulator: the thread issuing MMAs runs only about one MMA
+//               ahead of the tensor pipe, so a single issuer idles it while
+//               it waits for the next tile's operands and accumulator and
+//               while it commits.  One issuer behind a gate warp (which
+//               polled for it and cost two barrier hops a tile) took 2,130
+//               cycles a 128 x 256 x 144 tile, two issuers take 1,800 (1,152
+//               of MMA); 1,500 -> 1,450 at 64 columns, where the epilogue
+//               bounds the tile.  At 1M x 128 the clock falls with the busier
+//               pipe (the call is then bound by power), so the screen gains
+//               2%; 200,003 x 8: 2.01 -> 1.93 ms, 60,000 x 784 (one issuer,
+//               no gate): 1.06 -> 0.99 ms.
+//               Where the ring holds less than two tiles the first issuer
+//               issues all, each block as it lands.
 //   warps 2..   EW epilogue warps.  Warp w reads TMEM lane group w % 4 (the
 //               hardware's rule); the EW / 4 warps of a lane group take
 //               equal column ranges of each tile (16 warps for k <= 16, 8 for
@@ -34,7 +38,7 @@
 //               chunk: tcgen05.ld (two loads in flight), 3-input min over
 //               8-column groups, and only when a group passes the row's
 //               threshold, admit its columns (sinks.cuh).  The accumulator is
-//               handed back to the MMA warp as soon as its last chunk is in
+//               handed back to the issuers as soon as its last chunk is in
 //               registers.  The distance tile never reaches HBM.
 // A work unit is (query tile of 128 rows, split s of the reference tiles);
 // units are numbered split-major and claimed in order by the persistent CTAs
@@ -69,7 +73,7 @@ namespace {
 struct TcParams {
   uint32_t spin_limit;       // polls of a main-loop wait before it gives up
   int stages;
-  int a_blocks;              // 64-column query blocks the resident A region holds
+  int a_blocks;              // 64-column blocks of the launch's widest problem
   int m_tiles, S;            // single problem: m_tiles * S units, dealt round-robin
   const TcProblem* probs;    // batched: problem table
   const int4* items;         // batched: (problem, query tile, first tile, end tile)
@@ -100,7 +104,7 @@ constexpr int kUnitRing = 4;
 struct UnitRing {
   int* idx;          // [kUnitRing]
   uint64_t* full;    // [kUnitRing] producer -> consumers
-  uint64_t* empty;   // [kUnitRing] consumers (MMA thread + epilogue threads) -> producer
+  uint64_t* empty;   // [kUnitRing] consumers (MMA issuers + epilogue threads) -> producer
 };
 
 // The sequence of work units of this CTA; every warp role walks it in step.
@@ -192,12 +196,7 @@ constexpr uint32_t kATileBytes = kTcBM * kTcBK * 2;     // 16 KB per 64-column b
 constexpr uint32_t kBTileBytes = kTcBN * kTcBK * 2;     // 32 KB per 64-column block
 constexpr uint32_t kAAugBytes = kTcBM * kTcAug * 2;     // 4 KB (query ones)
 constexpr uint32_t kBAugBytes = kTcBN * kTcAug * 2;     // 8 KB (reference norms)
-constexpr int kSpillStride = 9;
-// go barriers (gate -> MMA issuer), used in turn by successive chunks: the gate
-// runs at most `stages` chunks (each at least one stage) ahead of the MMA
-// issuer, so with more barriers than the deepest ring a barrier's next phase
-// never starts before the issuer has consumed the previous one.
-constexpr int kGoRing = 16;  // 8 spilled values per thread, conflict-free stride
+constexpr int kSpillStride = 9;  // 8 spilled values per thread, conflict-free stride
 // A CTA allocates all 512 TMEM columns, so no two may share an SM: ask for at
 // least this much shared memory (more than half of the SM's 228 KB).
 constexpr size_t kMinCtaSmem = 116 * 1024;
@@ -209,7 +208,7 @@ __host__ __device__ inline uint32_t tc_stage_bytes(bool a_stream) {
 __host__ __device__ inline size_t tc_smem_bytes(int KB, int stages, bool a_stream, int ew) {
   size_t a = a_stream ? 0 : (size_t)KB * kATileBytes;
   size_t spill = (size_t)ew * 32 * kSpillStride * sizeof(float);
-  size_t bars = (2 * (size_t)stages + 8 + kGoRing + 2 * kUnitRing) * sizeof(uint64_t) + 16 +
+  size_t bars = (2 * (size_t)stages + 9 + 2 * kUnitRing) * sizeof(uint64_t) + 16 +
                 kUnitRing * sizeof(int);
   return 1024 /*alignment slack*/ + kAAugBytes + a + (size_t)tc_stage_bytes(a_stream) * stages +
          spill + bars;
@@ -228,7 +227,7 @@ B2K_DEV uint64_t smem_desc_sw32(const void* smem_tile) {
   return desc;
 }
 
-// Threads per CTA: producer warp, MMA warp, EW epilogue warps, gate warp.
+// Threads per CTA: producer warp, MMA issuer, EW epilogue warps, MMA issuer.
 __host__ __device__ constexpr int tc_block_threads(int ew) { return 96 + 32 * ew; }
 
 // Operand kinds of the screen kernel.
@@ -263,10 +262,9 @@ __global__ void __launch_bounds__(tc_block_threads(EW), 1)
   uint64_t* acc_full = a_empty + 1;   // [2]
   uint64_t* acc_empty = acc_full + 2; // [2]
   uint64_t* aaug_full = acc_empty + 2;
-  uint64_t* mma_drain = aaug_full + 1;  // the MMA issuer's exit: all its MMAs complete
-  uint64_t* go = mma_drain + 1;       // [kGoRing] gate -> MMA issuer, one per chunk in turn
+  uint64_t* mma_drain = aaug_full + 1;  // [2] an issuer's exit: all its MMAs complete
   UnitRing ring;
-  ring.full = go + kGoRing;            // [kUnitRing]
+  ring.full = mma_drain + 2;           // [kUnitRing]
   ring.empty = ring.full + kUnitRing;  // [kUnitRing]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ring.empty + kUnitRing);
   ring.idx = reinterpret_cast<int*>(tmem_slot + 4);
@@ -282,8 +280,8 @@ __global__ void __launch_bounds__(tc_block_threads(EW), 1)
       mbar_init(&empty[s], 1);
     }
     mbar_init(a_full, 1);
-    // the query tile is free once its unit's MMAs are done (MMA commit) and
-    // its load has landed (gate; a unit may have no tiles at all)
+    // the query tile is free once both issuers' MMAs of its unit are done (each
+    // commits after it has seen the load land; a unit may have no tiles at all)
     mbar_init(a_empty, 2);
     mbar_init(&acc_full[0], 1);
     mbar_init(&acc_full[1], 1);
@@ -292,11 +290,11 @@ __global__ void __launch_bounds__(tc_block_threads(EW), 1)
     mbar_init(&acc_empty[0], EW);
     mbar_init(&acc_empty[1], EW);
     mbar_init(aaug_full, 1);
-    mbar_init(mma_drain, 1);
-    for (int g = 0; g < kGoRing; ++g) mbar_init(&go[g], 1);
+    mbar_init(&mma_drain[0], 1);
+    mbar_init(&mma_drain[1], 1);
     for (int r = 0; r < kUnitRing; ++r) {
       mbar_init(&ring.full[r], 1);
-      mbar_init(&ring.empty[r], 2 + kEpiThreads);  // MMA issuer, gate, epilogue threads
+      mbar_init(&ring.empty[r], 2 + kEpiThreads);  // MMA issuers, epilogue threads
     }
     fence_mbar_init();
   }
@@ -380,7 +378,7 @@ __global__ void __launch_bounds__(tc_block_threads(EW), 1)
           phase ^= 1;
         }
       }
-      // with claimed units the MMA warp releases the query tile after every
+      // with claimed units the issuers release the query tile after every
       // unit: take the last release so no arrival lands after the CTA exits
       if (!A_STREAM && cur.dyn) mbar_wait(a_empty, a_phase ^ 1, status, DEV_TIMEOUT_A, lim);
     prod_done:
@@ -392,9 +390,10 @@ __global__ void __launch_bounds__(tc_block_threads(EW), 1)
       if (a_loads) mbar_wait_drain(a_full, (a_loads - 1) & 1u, status);
       mbar_wait_drain(aaug_full, 0, status);
     }
-  } else if (warp == 1) {
-    // --------------------------------------------------------- MMA issuer
+  } else if (warp == 1 || warp == 2 + EW) {
+    // -------------------------------------------------------- MMA issuers
     if (lane == 0) {
+      const uint32_t mine = warp == 1 ? 0u : 1u;  // accumulator of this issuer's tiles
       constexpr uint32_t idesc = TF32 ? idesc_tf32(kTcBM, kTcBN)
                                  : U8 ? idesc_u8(kTcBM, kTcBN)
                                       : idesc_f16(kTcBM, kTcBN, 1);
@@ -407,97 +406,95 @@ __global__ void __launch_bounds__(tc_block_threads(EW), 1)
         else
           mma_f16(d_tmem, a, b, idesc, acc);
       };
-      uint32_t stage = 0, acc_it = 0, chunk = 0;
+      // operand descriptors of stage 0 (and of the resident query blocks); a
+      // stage or block on is an addition to the address field (16-byte units)
+      const uint64_t a_desc = smem_desc_sw128(A_STREAM ? b_smem : a_smem);
+      const uint64_t b_desc = smem_desc_sw128(b_smem + b_off);
+      const uint64_t aug_desc = smem_desc_sw32(b_smem + baug_off);
+      const uint64_t ones_desc = smem_desc_sw32(aaug_smem);
+      const uint32_t step = stage_bytes >> 4;
+      // tiles alternate between the issuers when the ring holds two of them
+      // (of the launch's widest problem); else the first issues all
+      const bool pair = 2 * p.a_blocks <= nst;
+      uint32_t stage = 0, phase = 0, a_phase = 0, tile = 0;
       bool issued = false;  // any MMA (for the exit path's drain)
+      auto advance = [&](uint32_t by) {
+        stage += by;
+        while (stage >= (uint32_t)nst) {
+          stage -= nst;
+          phase ^= 1;
+        }
+      };
+      if (!mbar_wait(aaug_full, 0, status, DEV_TIMEOUT_A, lim)) goto mma_done;
       {
-        const uint64_t aaug_desc = smem_desc_sw32(aaug_smem);
         UnitCursor<BATCH> cur(p, ring, false);
         TcUnit x;
         while (cur.next(p, x)) {
           const int KB = x.pr->KB;
-          const int C = max(1, min(KB, nst / 2));  // blocks per gated chunk
-          for (int j = x.j0; j < x.j1; ++j) {
-            const uint32_t buf = acc_it & 1;
+          bool any = false;
+          if (!A_STREAM) {
+            if (!mbar_wait(a_full, a_phase, status, DEV_TIMEOUT_A, lim)) goto mma_done;
+            a_phase ^= 1;
+          }
+          for (int j = x.j0; j < x.j1; ++j, ++tile) {
+            const uint32_t buf = tile & 1;
+            if (pair ? buf != mine : mine != 0) {  // the other issuer's tile
+              advance(KB);
+              continue;
+            }
             const uint32_t d_tmem = tmem_base + buf * kTcBN;
-            for (int kb = 0; kb < KB; ++kb) {
-              if (kb % C == 0) {
-                // the chunk's operands are in shared memory (and, at kb 0, the
-                // accumulator is free)
-                if (!mbar_wait(&go[chunk % kGoRing], (chunk / kGoRing) & 1, status,
-                               DEV_TIMEOUT_ACC, lim))
-                  goto mma_done;
-                ++chunk;
-                tc_fence_after();
+            // the epilogue has read this accumulator's previous tile (so every
+            // tile up to that one was loaded: with pairs, no stage below is
+            // more than one phase ahead of its barrier)
+            if (!mbar_wait(&acc_empty[buf], ((tile >> 1) & 1) ^ 1, status, DEV_TIMEOUT_ACC, lim))
+              goto mma_done;
+            if (pair) {
+              uint32_t s = stage, ph = phase;
+              for (int kb = 0; kb < KB; ++kb) {
+                if (!mbar_wait(&full[s], ph, status, DEV_TIMEOUT_FULL, lim)) goto mma_done;
+                if (++s == (uint32_t)nst) {
+                  s = 0;
+                  ph ^= 1;
+                }
               }
-              issued = true;
-              uint8_t* st = b_smem + (size_t)stage * stage_bytes;
-              const uint8_t* a_tile = A_STREAM ? st : a_smem + kb * kATileBytes;
-              const uint64_t adesc = smem_desc_sw128(a_tile);
-              const uint64_t bdesc = smem_desc_sw128(st + b_off);
+            }
+            issued = any = true;
+            for (int kb = 0; kb < KB; ++kb) {
+              if (!pair && !mbar_wait(&full[stage], phase, status, DEV_TIMEOUT_FULL, lim))
+                goto mma_done;
+              tc_fence_after();
+              const uint32_t off = stage * step;
+              const uint64_t ad = A_STREAM ? a_desc + off : a_desc + kb * (kATileBytes >> 4);
+              const uint64_t bd = b_desc + off;
 #pragma unroll
               for (int kk = 0; kk < 4; ++kk) {
                 // advance 32 bytes inside the 128-byte swizzle atom: +2 in 16-byte units
-                mma(d_tmem, adesc + 2 * kk, bdesc + 2 * kk, (kb | kk) != 0);
+                mma(d_tmem, ad + 2 * kk, bd + 2 * kk, (kb | kk) != 0);
               }
               if (!U8 && kb == KB - 1)  // + ||y_x||^2 through the norm columns
-                mma(d_tmem, aaug_desc, smem_desc_sw32(st + baug_off), 1);
+                mma(d_tmem, ones_desc, aug_desc + off, 1);
               mma_commit(&empty[stage]);
-              if (++stage == (uint32_t)nst) stage = 0;
+              advance(1);
             }
             mma_commit(&acc_full[buf]);
-            ++acc_it;
           }
           // Release the query tile for the next unit (not after the last one, so
           // no arrival can land after the CTA has exited).
-          if (!A_STREAM && cur.more()) mma_commit(a_empty);
+          if (!A_STREAM && cur.more()) {
+            if (any)
+              mma_commit(a_empty);
+            else
+              mbar_arrive(a_empty);
+          }
         }
       }
     mma_done:
       // every MMA this thread issued has completed before the CTA moves on to
       // free its TMEM (on the normal path the epilogue has seen them all)
       if (issued) {
-        mma_commit(mma_drain);
-        mbar_wait_drain(mma_drain, 0, status);
+        mma_commit(&mma_drain[mine]);
+        mbar_wait_drain(&mma_drain[mine], 0, status);
       }
-    }
-  } else if (warp == 2 + EW) {
-    // --------------------------------------------------------------- gate
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0, a_phase = 0, acc_it = 0, chunk = 0;
-      if (!mbar_wait(aaug_full, 0, status, DEV_TIMEOUT_A, lim)) goto gate_done;
-      {
-        UnitCursor<BATCH> cur(p, ring, false);
-        TcUnit x;
-        while (cur.next(p, x)) {
-          const int KB = x.pr->KB;
-          const int C = max(1, min(KB, nst / 2));  // as the MMA issuer
-          if (!A_STREAM) {
-            if (!mbar_wait(a_full, a_phase, status, DEV_TIMEOUT_A, lim)) goto gate_done;
-            a_phase ^= 1;
-          }
-          for (int j = x.j0; j < x.j1; ++j) {
-            const uint32_t buf = acc_it & 1, apar = (acc_it >> 1) & 1;
-            // the epilogue has read this buffer's previous tile
-            if (!mbar_wait(&acc_empty[buf], apar ^ 1, status, DEV_TIMEOUT_ACC, lim))
-              goto gate_done;
-            for (int kb = 0; kb < KB; ++kb) {
-              if (!mbar_wait(&full[stage], phase, status, DEV_TIMEOUT_FULL, lim)) goto gate_done;
-              if (++stage == (uint32_t)nst) {
-                stage = 0;
-                phase ^= 1;
-              }
-              if ((kb + 1) % C == 0 || kb + 1 == KB) {
-                mbar_arrive(&go[chunk % kGoRing]);
-                ++chunk;
-              }
-            }
-            ++acc_it;
-          }
-          // (not after the last unit, as with the MMA issuer's release)
-          if (!A_STREAM && cur.more()) mbar_arrive(a_empty);
-        }
-      }
-    gate_done:;
     }
   } else {
     // ----------------------------------------------------------- epilogue
@@ -688,7 +685,7 @@ int launch_tc_variant(const TcMapSet<BATCH ? kBatchGroups : 1>& maps, const TcPa
 // each group keeps its own candidate lists.
 // Epilogue warps of the single-problem kNN screen: four per TMEM lane group
 // for the register-heap trackers (k <= 16), which shortens each warp's
-// per-tile chain and cuts the MMA warp's waits for a free accumulator
+// per-tile chain and cuts the issuers's waits for a free accumulator
 // (B2K_TC_EW=8 selects two); two for the lazy tracker.
 static int tc_knn_ew(int k) {
   if (k > 16) return 8;

@@ -713,9 +713,18 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
       // of the query, so it is >= the final V_k and the certificate holds.
       const int64_t m_tiles = m_pad / kTcBM;
       const int kSeedTiles = seed_tiles();
-      if (key && ix.group_start && !tc_lazy_sink(k) && n_tiles >= 2 * kSeedTiles &&
-          seed_enabled()) {
-        const int G = tc_column_groups(k);
+      //
+      // For k > 16 the pass runs the register tracker at its widest, 16 values
+      // in each of four column groups, and launch_seed_kth takes the k-th
+      // smallest of those 64: the k-th smallest of some of the query's values
+      // is no smaller than that of all.  60,013 x 100 rows against themselves,
+      // k = 50: list entries 88M -> 37M, screen 5.71 -> 2.38 ms (1.79 with
+      // sixteen epilogue warps).  Filling the lazy tracker's own lists in the
+      // pass instead cost 2.3 ms, the pass itself 0.45.
+      const bool lazy = tc_lazy_sink(k);
+      if (key && ix.group_start && n_tiles >= 2 * kSeedTiles && seed_enabled()) {
+        const int ks = lazy ? 16 : k;
+        const int G = tc_column_groups(ks);
         int* home = nullptr;
         int* seed_counts = nullptr;
         float* seed_kth = nullptr;
@@ -723,7 +732,7 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
         fr.keep(home);
         if ((rc = dalloc(&seed_counts, (size_t)G * m_pad, st))) return rc;
         fr.keep(seed_counts);
-        if ((rc = dalloc(&seed_kth, (size_t)G * m_pad * k, st))) return rc;
+        if ((rc = dalloc(&seed_kth, (size_t)G * m_pad * ks, st))) return rc;
         fr.keep(seed_kth);
         launch_home_tiles(perm, key, m, ix.group_start, (int)n_tiles, kSeedTiles, home,
                           (int)m_tiles, st);
@@ -731,12 +740,15 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
         sb.out.cap = 0;  // the trackers only: no list entry is written
         sb.out.counts = seed_counts;
         sb.out.kth = seed_kth;
+        sb.k = ks;
+        if (lazy) sb.shared_kth = nullptr;  // a group's 16th value is not the query's k-th
         // status[7] (zeroed above) counts this pass's claimed units
         int lr = launch_screen_tc(&ix, &tmap_a, m, m_pad, exclude_self, q_offset, 1, qp.E,
                                   kSinkKnn, sb, status, st, perm, status + 7, tf32, home,
                                   kSeedTiles);
         if (lr) return fail(B2K_ECUDA, "tcgen05 seeding screen launch failed: %s",
                             cudaGetErrorString((cudaError_t)lr));
+        if (lazy && G * ks >= k) launch_seed_kth(seed_kth, G, ks, m, m_pad, k, shared_kth, st);
         if (stats) cudaEventRecord(ev[4], st);
         seeded = true;
       }
@@ -775,6 +787,7 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
     ca.status = status;
     ca.nq = qp.nq;
     ca.refined = counters + 4;
+    ca.shared_kth = shared_kth;
     launch_certify(ca, st);
     B2K_CUDA(cudaGetLastError());
     // Rows the screen could not certify (a list past capacity, too many

@@ -237,6 +237,11 @@ void launch_assign_rows(const Index* ix, const float* X, int64_t n, int* key, in
 void launch_home_tiles(const int* perm, const int* key, int64_t m, const int* group_start,
                        int n_tiles, int window, int* home, int m_tiles, cudaStream_t st);
 
+// shared_kth[r] = the k-th smallest of query r's values in `groups` (<= 4) ascending
+// lists of kl, kth [groups][m_pad][kl] (unchanged when fewer than k are finite)
+void launch_seed_kth(const float* kth, int groups, int kl, int64_t m, int64_t m_pad, int k,
+                     uint32_t* shared_kth, cudaStream_t st);
+
 // second pass over uncertified rows: Qout[i] = Qs[rows[i]], pout[i] = perm[rows[i]]
 void launch_gather_fallback(const float* Qs, int d, const int* rows, const int* perm, int count,
                             float* Qout, int* pout, cudaStream_t st);
@@ -261,6 +266,7 @@ struct CertifyArgs {
   const int* status;   // error word of the call: nonzero (a screen gave up) = do nothing
   const double* nq;    // [m] ||q - center||^2 (float64): enables the two-stage refine, or null
   unsigned long long* refined;  // candidates refined in fp32 (counter), or null
+  const uint32_t* shared_kth;  // [m] the screen's final shared k-th keys, or null
 };
 void launch_certify(const CertifyArgs& a, cudaStream_t st);
 // problem p owns global rows [row_start[p], row_start[p + 1]) of the batch

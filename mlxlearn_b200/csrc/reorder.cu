@@ -22,6 +22,7 @@
 
 #include "common.cuh"
 #include "internal.cuh"
+#include "tracker.cuh"
 
 namespace b2k {
 
@@ -234,7 +235,46 @@ __global__ void home_tiles_kernel(const int* __restrict__ perm, const int* __res
   home[t] = max(j0, 0);
 }
 
+// One thread per query: the k-th smallest of its G ascending lists of kl values
+// (a k-way merge by list heads) as its shared k-th key; a query with fewer than
+// k finite values keeps its key.
+__global__ void seed_kth_kernel(const float* __restrict__ kth, int G, int kl, int64_t m,
+                                int64_t m_pad, int k, uint32_t* __restrict__ shared_kth) {
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= m) return;
+  constexpr int kMaxG = 4;
+  float head[kMaxG];
+  int pos[kMaxG];
+#pragma unroll
+  for (int g = 0; g < kMaxG; ++g) {
+    pos[g] = 0;
+    head[g] = g < G ? kth[((size_t)g * m_pad + r) * kl] : INFINITY;
+  }
+  float v = INFINITY;
+  for (int t = 0; t < k; ++t) {
+    int b = 0;
+#pragma unroll
+    for (int g = 1; g < kMaxG; ++g)
+      if (head[g] < head[b]) b = g;
+#pragma unroll
+    for (int g = 0; g < kMaxG; ++g)
+      if (g == b) {
+        v = head[g];
+        ++pos[g];
+        head[g] = pos[g] < kl ? kth[((size_t)g * m_pad + r) * kl + pos[g]] : INFINITY;
+      }
+  }
+  if (v < INFINITY) shared_kth[r] = float_key(v);
+}
+
 }  // namespace
+
+void launch_seed_kth(const float* kth, int groups, int kl, int64_t m, int64_t m_pad, int k,
+                     uint32_t* shared_kth, cudaStream_t st) {
+  if (m <= 0) return;
+  seed_kth_kernel<<<(unsigned)((m + 127) / 128), 128, 0, st>>>(kth, groups, kl, m, m_pad, k,
+                                                               shared_kth);
+}
 
 void launch_home_tiles(const int* perm, const int* key, int64_t m, const int* group_start,
                        int n_tiles, int window, int* home, int m_tiles, cudaStream_t st) {

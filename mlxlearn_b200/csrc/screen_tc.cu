@@ -33,8 +33,7 @@
 //               issues all, each block as it lands.
 //   warps 2..   EW epilogue warps.  Warp w reads TMEM lane group w % 4 (the
 //               hardware's rule); the EW / 4 warps of a lane group take
-//               equal column ranges of each tile (16 warps for k <= 16, 8 for
-//               the lazy tracker).  Per 32-column
+//               equal column ranges of each tile.  Per 32-column
 //               chunk: tcgen05.ld (two loads in flight), 3-input min over
 //               8-column groups, and only when a group passes the row's
 //               threshold, admit its columns (sinks.cuh).  The accumulator is
@@ -683,12 +682,14 @@ int launch_tc_variant(const TcMapSet<BATCH ? kBatchGroups : 1>& maps, const TcPa
 
 // Column groups (epilogue warps per TMEM lane group) of the kNN screen for k:
 // each group keeps its own candidate lists.
-// Epilogue warps of the single-problem kNN screen: four per TMEM lane group
-// for the register-heap trackers (k <= 16), which shortens each warp's
-// per-tile chain and cuts the issuers's waits for a free accumulator
-// (B2K_TC_EW=8 selects two); two for the lazy tracker.
+// Epilogue warps of the single-problem kNN screen: four per TMEM lane group,
+// which shortens each warp's per-tile chain and cuts the issuers' waits for a
+// free accumulator (B2K_TC_EW=8 selects two).  The lazy tracker (k > 16) gains
+// twice: its lists hold kListCap entries each, so four a split also keep rows
+// whose certified band is wide from compacting at every chunk (1M x 128, 20,000
+// queries, k = 50: 216 ms with eight warps, 6.4 with sixteen; 200,000 x 64,
+// k = 32: 3.37 and 2.16).
 static int tc_knn_ew(int k) {
-  if (k > 16) return 8;
   static const int ew = [] {
     const char* e = getenv("B2K_TC_EW");
     return (e && atoi(e) == 8) ? 8 : 16;
@@ -742,7 +743,8 @@ int launch_screen_tc(Index* ix, const CUtensorMap* tmap_a, int64_t m, int64_t m_
     if (tc_knn_ew(sa.k) == 16) {
       if (sa.k <= 8) return B2K_TC_LAUNCH_TF32(KnnSink<8>, 16);
       if (sa.k <= 12) return B2K_TC_LAUNCH_TF32(KnnSink<12>, 16);
-      return B2K_TC_LAUNCH_TF32(KnnSink<16>, 16);
+      if (!tc_lazy_sink(sa.k)) return B2K_TC_LAUNCH_TF32(KnnSink<16>, 16);
+      return B2K_TC_LAUNCH_TF32(LazyKnnSink, 16);
     }
     if (sa.k <= 8) return B2K_TC_LAUNCH_TF32(KnnSink<8>, 8);
     if (sa.k <= 12) return B2K_TC_LAUNCH_TF32(KnnSink<12>, 8);
@@ -759,7 +761,8 @@ int launch_screen_tc(Index* ix, const CUtensorMap* tmap_a, int64_t m, int64_t m_
   if (tc_knn_ew(sa.k) == 16) {
     if (sa.k <= 8) return B2K_TC_LAUNCH(KnnSink<8>, 16);
     if (sa.k <= 12) return B2K_TC_LAUNCH(KnnSink<12>, 16);
-    return B2K_TC_LAUNCH(KnnSink<16>, 16);
+    if (!tc_lazy_sink(sa.k)) return B2K_TC_LAUNCH(KnnSink<16>, 16);
+    return B2K_TC_LAUNCH(LazyKnnSink, 16);
   }
   if (sa.k <= 8) return B2K_TC_LAUNCH(KnnSink<8>, 8);
   if (sa.k <= 12) return B2K_TC_LAUNCH(KnnSink<12>, 8);

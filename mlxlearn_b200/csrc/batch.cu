@@ -449,6 +449,7 @@ int build_tuned(b2k_batch* b, const std::map<TuneKey, Tuning>& tune, int gran,
       c.scr = so;
       c.E = b->E + p.pad0;
       c.nq = b->nq + p.pad0;  // two-stage refinement (certify.cu)
+      c.shared_kth = b->skth + p.pad0;
       c.dist = p.dist;
       c.idx = p.idx;
       c.fallback_list = b->fb_list;

@@ -24,6 +24,7 @@
 // (src/mlxlearn_device/_neighbors_fused.py:545-834,
 //  _neighbors_shortlist.py:16-170, _neighbors_precision.py:9-259) and its
 // partitioned exact fallback (_neighbors_fallback.py:62-298).
+#include <algorithm>
 #include <cfloat>
 
 #include "common.cuh"
@@ -35,6 +36,26 @@ namespace b2k {
 namespace {
 
 constexpr int kCertWarps = 8;
+// Rows a block of a batch takes, its warps one at a time as they finish: rows
+// differ in candidates by up to 100x, and with one row a warp a block holds its
+// shared memory until the slowest is done (11 of 16 warps resident).  32 uneven
+// problems: 1.49 ms with 8 rows a block, 1.38 with 16, 1.33 with 24.  A single
+// index keeps one row a warp: its consecutive (grouped) rows share neighbours,
+// and the closer in time they run the better L1 and L2 hold those (100,000
+// queries of 1M x 128: 2.33 ms with 8, 2.48 with 16, 2.75 with 24; 60,000 x
+// 784: 254, 285, 291 us).  Few rows spread over the SMs first.
+constexpr int kCertBatchRows = 24;
+inline int cert_batch_rows(int64_t rows) {
+  const int64_t spread = (rows + 1183) / 1184;  // about eight blocks an SM
+  return (int)std::min<int64_t>(kCertBatchRows,
+                                (spread + kCertWarps - 1) / kCertWarps * kCertWarps);
+}
+// Up to this many candidates go straight to their float64 values (one round of
+// the warp): the fp32 refinement and its selects cost more than they drop.
+// With the lists walked as one, the shared bound and this: 60,013 x 100 against
+// itself, k = 50: 2.10 -> 1.60 ms; 200,003 x 8, 50,021 queries: 0.39 -> 0.20 ms.
+constexpr int kDirectCandidates = 32;
+constexpr int kFlatLists = 256;    // lists walked as one concatenation (offsets in the histogram)
 constexpr int kSurvivorCap = 256;  // candidates that can still reach the top k
 constexpr size_t kCertWarpBytes =
     (size_t)kCertifyCap * (sizeof(int) + sizeof(float)) +
@@ -93,9 +114,14 @@ __device__ unsigned warp_sort_resolve(double* s, int* id, int C, int k, const fl
   __syncwarp();
   warp_bitonic(s, id, P, lane);
   unsigned compares = 0;
+  const double g2 = interval_g2(d);
+  const double lo_f = 1.0 - g2, hi_f = 1.0 + g2;
+  // neighbours whose intervals overlap, all lanes at once: mostly none
+  bool near = false;
+  for (int i = lane; i < k && i + 1 < C; i += 32)
+    near |= __dmul_rd(s[i + 1], lo_f) <= __dmul_ru(s[i], hi_f);
+  if (!__any_sync(0xffffffffu, near)) return 0;
   if (lane == 0) {
-    const double g2 = interval_g2(d);
-    const double lo_f = 1.0 - g2, hi_f = 1.0 + g2;
     int i = 0;
     while (i < k && i < C) {
       int j = i + 1;
@@ -394,27 +420,135 @@ __device__ __forceinline__ void certify_row(const CertifyArgs& a, int64_t row, u
     if (__shfl_sync(0xffffffffu, st, 0) != DEV_OK) return;
   }
 
-  // 1. overflow check
+  // 1. overflow check; the lists' offsets in their concatenation (`hist`,
+  // until a radix select needs it)
   bool overflow = false;
   unsigned entries = 0;
-  for (int s = lane; s < S; s += 32) {
-    int c = so.counts[(size_t)s * so.m_pad + row];
+  const bool flat = S <= kFlatLists;
+  for (int s0 = 0; s0 < S; s0 += 32) {
+    const int s = s0 + lane;
+    const int c = s < S ? so.counts[(size_t)s * so.m_pad + row] : 0;
     overflow |= c > so.cap;
-    entries += c;
+    unsigned incl = (unsigned)c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    if (flat && s < S) hist[s] = entries + incl - (unsigned)c;
+    entries += __shfl_sync(0xffffffffu, incl, 31);
   }
   overflow = __any_sync(0xffffffffu, overflow);
   if (overflow) {
     if (lane == 0) a.fallback_list[atomicAdd(a.fallback_count, 1)] = (int)(a.row_base + row);
     return;
   }
-  entries = __reduce_add_sync(0xffffffffu, entries);
+  __syncwarp();
+  // Entries with v <= limit into (ci, cv), up to kCertifyCap; returns how many
+  // there are (counting stops past the capacity).  Four entries a lane in
+  // flight: the loop is bound by their latency.  Short lists are walked as one
+  // concatenation (each entry finds its list by bisection of the offsets): list
+  // by list, a row of 20 lists of 30 entries spent 20 dependent round trips on
+  // 5 rounds of work, and a single query's 160 lists 96 us of a 194 us call.
+  constexpr int kAhead = 4;
+  auto gather = [&](float limit) -> int {
+    int C = 0;
+    auto take = [&](const int2(&e)[kAhead], const bool(&in)[kAhead]) {
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const float v = __int_as_float(e[u].x);
+        const bool pass = in[u] && v <= limit;
+        const unsigned bal = __ballot_sync(0xffffffffu, pass);
+        const int pos = C + __popc(bal & ((1u << lane) - 1));
+        if (pass && pos < kCertifyCap) {
+          ci[pos] = e[u].y;
+          cv[pos] = v;  // the screen value until the refinement overwrites it
+        }
+        C += __popc(bal);
+      }
+    };
+    if (flat && entries < 64u * (unsigned)S) {
+      for (unsigned base = 0; base < entries && C <= kCertifyCap; base += 32 * kAhead) {
+        int2 e[kAhead];
+        bool in[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          const unsigned i = base + 32 * u + lane;
+          in[u] = i < entries;
+          e[u] = make_int2(0, 0);
+          if (in[u]) {
+            int lo = 0, hi = S - 1;  // the last list whose offset is <= i
+            while (lo < hi) {
+              const int mid = (lo + hi + 1) >> 1;
+              if (hist[mid] <= i)
+                lo = mid;
+              else
+                hi = mid - 1;
+            }
+            e[u] = so.lists[((size_t)lo * so.m_pad + row) * so.cap + (i - hist[lo])];
+          }
+        }
+        take(e, in);
+      }
+      return C;
+    }
+    for (int s = 0; s < S && C <= kCertifyCap; ++s) {
+      const size_t slot = (size_t)s * so.m_pad + row;
+      const int cnt = so.counts[slot];
+      const int2* lst = so.lists + slot * so.cap;
+      for (int base = 0; base < cnt && C <= kCertifyCap; base += 32 * kAhead) {
+        int2 e[kAhead];
+        bool in[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          const int i = base + 32 * u + lane;
+          in[u] = i < cnt;
+          e[u] = in[u] ? lst[i] : make_int2(0, 0);
+        }
+        take(e, in);
+      }
+    }
+    return C;
+  };
+  const float E2 = __fmul_ru(2.0f, a.E[row]);
 
   // 2. V_k = k-th smallest of the lists' k smallest values (radix select);
   // screens without per-slot k-th values list every value up to their own
-  // threshold, which covers the k smallest overall: select over the lists.
+  // threshold, which covers the k smallest overall.  There the final shared
+  // k-th value B >= V_k cuts the lists first: the entries with v <= B + 2E hold
+  // the k smallest and every candidate, so V_k is selected among them in shared
+  // memory and the candidates are compacted in place (one pass over the lists
+  // instead of five).
   const int total = S * k;
   float Vk;
-  if (!so.kth) {
+  int C = -1;  // candidates, once gathered
+  const uint32_t bound_key = (!so.kth && a.shared_kth) ? a.shared_kth[row] : 0xffffffffu;
+  if (bound_key != 0xffffffffu && (C = gather(__fadd_ru(key_float(bound_key), E2))) >= k &&
+      C <= kCertifyCap) {
+    __syncwarp();
+    auto value_key = [&](int c) { return float_key(cv[c]); };
+    Vk = key_float(C <= 32 ? warp_kth_32(lane < C ? value_key(lane) : 0u, C, k, lane)
+                           : warp_radix_kth(value_key, C, k, hist, lane));
+    __syncwarp();
+    const float Tc = __fadd_ru(Vk, E2);
+    int w = 0;
+    for (int base = 0; base < C; base += 32) {
+      const int c = base + lane;
+      const float v = c < C ? cv[c] : 0.0f;
+      const int col = c < C ? ci[c] : 0;
+      const bool keep = c < C && v <= Tc;
+      // every lane has read its entry before any write
+      const unsigned bal = __ballot_sync(0xffffffffu, keep);
+      if (keep) {
+        const int p = w + __popc(bal & ((1u << lane) - 1));
+        cv[p] = v;
+        ci[p] = col;
+      }
+      w += __popc(bal);
+    }
+    C = w;
+  } else if (!so.kth) {
+    C = -1;
     Vk = key_float(warp_radix_select(
         [&](auto f) {
           for (int s = 0; s < S; ++s) {
@@ -465,41 +599,30 @@ __device__ __forceinline__ void certify_row(const CertifyArgs& a, int64_t row, u
         },
         total, k, hist, lane));
   }
-  const float Tf = __fadd_ru(Vk, __fmul_ru(2.0f, a.E[row]));
-
-  // 3. gather candidates v <= Tf.  Each lane keeps four list entries in
-  // flight (the loop is bound by their latency), and the columns of grouped
-  // operand rows are mapped to training rows afterwards, all at once.
-  int C = 0;
-  bool too_many = false;
-  constexpr int kAhead = 4;
-  for (int s = 0; s < S && !too_many; ++s) {
-    const size_t slot = (size_t)s * so.m_pad + row;
-    const int cnt = so.counts[slot];
-    const int2* lst = so.lists + slot * so.cap;
-    for (int base = 0; base < cnt && !too_many; base += 32 * kAhead) {
-      int2 e[kAhead];
+  // 3. candidates: entries v <= V_k + 2E.  The columns of grouped operand rows
+  // are mapped to training rows afterwards, all at once.  (A radix select above
+  // has used `hist`: the offsets are formed again.)
+  if (C < 0) {
+    if (flat) {
+      unsigned off = 0;
+      __syncwarp();
+      for (int s0 = 0; s0 < S; s0 += 32) {
+        const int s = s0 + lane;
+        const unsigned c = s < S ? (unsigned)so.counts[(size_t)s * so.m_pad + row] : 0u;
+        unsigned incl = c;
 #pragma unroll
-      for (int u = 0; u < kAhead; ++u) {
-        const int i = base + 32 * u + lane;
-        e[u] = i < cnt ? lst[i] : make_int2(0, 0);
-      }
-#pragma unroll
-      for (int u = 0; u < kAhead; ++u) {
-        const int i = base + 32 * u + lane;
-        const float v = __int_as_float(e[u].x);
-        const bool pass = i < cnt && v <= Tf;
-        const unsigned bal = __ballot_sync(0xffffffffu, pass);
-        const int pos = C + __popc(bal & ((1u << lane) - 1));
-        if (pass && pos < kCertifyCap) {
-          ci[pos] = e[u].y;
-          cv[pos] = v;  // the screen value until the refinement overwrites it
+        for (int o = 1; o < 32; o <<= 1) {
+          const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += t;
         }
-        C += __popc(bal);
+        if (s < S) hist[s] = off + incl - c;
+        off += __shfl_sync(0xffffffffu, incl, 31);
       }
-      too_many = C > kCertifyCap;
+      __syncwarp();
     }
+    C = gather(__fadd_ru(Vk, E2));
   }
+  const bool too_many = C > kCertifyCap;
   // grouped operand rows: the lists hold operand rows, the answer training rows
   if (!too_many && a.cols) {
     __syncwarp();
@@ -516,56 +639,75 @@ __device__ __forceinline__ void certify_row(const CertifyArgs& a, int64_t row, u
   const float g32 = (float)((double)(a.d + 5) * 0x1p-24 * 1.01);
   const float abs32 = (float)a.d * 0x1p-126f;
   const float up_f = 1.0f + g32, lo_f = 1.0f - g32;
-  float U0;
-  const int Cr = refine_candidates(a, row, q, ci, cv, si, reinterpret_cast<float*>(cs), hist, C,
-                                   up_f, abs32, Vk, &U0, lane);
-  // 5. U = k-th smallest upper bound.  After a two-stage refinement the
-  // stage-one candidates (among the refined) put k upper bounds at or below
-  // U0, so only those bounds can be the k-th smallest: when at most 32, a
-  // rank select among them; otherwise a radix select over all.
-  auto upper_key = [&](int c) { return float_key(__fadd_ru(__fmul_ru(cv[c], up_f), abs32)); };
-  uint32_t Ukey = 0;
-  bool small = false;
-  if (U0 < INFINITY) {
-    // the keys <= U0, gathered through the survivor scratch (free until step 6)
-    uint32_t* tmp = reinterpret_cast<uint32_t*>(si);
-    const uint32_t u0 = float_key(U0);
-    int n = 0;
-    for (int base = 0; base < Cr && n <= 32; base += 32) {
+  int Cr = 0, Cs = C;
+  if (C <= kDirectCandidates || 2 * C <= 3 * k) {
+    // few candidates, or nearly all of them answers: every one survives
+    for (int c = lane; c < C; c += 32) si[c] = ci[c];
+    __syncwarp();
+  } else {
+    float U0;
+    Cr = refine_candidates(a, row, q, ci, cv, si, reinterpret_cast<float*>(cs), hist, C,
+                                     up_f, abs32, Vk, &U0, lane);
+    // 5. U = k-th smallest upper bound.  After a two-stage refinement the
+    // stage-one candidates (among the refined) put k upper bounds at or below
+    // U0, so only those bounds can be the k-th smallest: when at most 32, a
+    // rank select among them; otherwise a radix select over all.
+    auto upper_key = [&](int c) { return float_key(__fadd_ru(__fmul_ru(cv[c], up_f), abs32)); };
+    uint32_t Ukey = 0;
+    bool small = false;
+    if (U0 < INFINITY) {
+      // the keys <= U0, gathered through the survivor scratch (free until step 6)
+      uint32_t* tmp = reinterpret_cast<uint32_t*>(si);
+      const uint32_t u0 = float_key(U0);
+      int n = 0;
+      for (int base = 0; base < Cr && n <= 32; base += 32) {
+        const int c = base + lane;
+        const uint32_t key = c < Cr ? upper_key(c) : 0xffffffffu;
+        const bool le = c < Cr && key <= u0;
+        const unsigned bal = __ballot_sync(0xffffffffu, le);
+        const int pos = n + __popc(bal & ((1u << lane) - 1));
+        if (le && pos < 32) tmp[pos] = key;
+        n += __popc(bal);
+      }
+      __syncwarp();
+      if (n <= 32 && n >= k) {
+        Ukey = warp_kth_32(lane < n ? tmp[lane] : 0u, n, k, lane);
+        small = true;
+      }
+      __syncwarp();
+    }
+    if (!small) Ukey = warp_radix_kth(upper_key, Cr, k, hist, lane);
+    const float U = key_float(Ukey);
+    // 6. survivors: lower bound <= U (everything that can still be in the top k)
+    Cs = 0;
+    for (int base = 0; base < Cr; base += 32) {
       const int c = base + lane;
-      const uint32_t key = c < Cr ? upper_key(c) : 0xffffffffu;
-      const bool le = c < Cr && key <= u0;
-      const unsigned bal = __ballot_sync(0xffffffffu, le);
-      const int pos = n + __popc(bal & ((1u << lane) - 1));
-      if (le && pos < 32) tmp[pos] = key;
-      n += __popc(bal);
+      const bool keep = c < Cr && __fsub_rd(__fmul_rd(cv[c], lo_f), abs32) <= U;
+      const unsigned bal = __ballot_sync(0xffffffffu, keep);
+      const int pos = Cs + __popc(bal & ((1u << lane) - 1));
+      if (keep && pos < kSurvivorCap) si[pos] = ci[c];
+      Cs += __popc(bal);
+    }
+    if (Cs > kSurvivorCap) {
+      if (lane == 0) a.fallback_list[atomicAdd(a.fallback_count, 1)] = (int)(a.row_base + row);
+      return;
     }
     __syncwarp();
-    if (n <= 32 && n >= k) {
-      Ukey = warp_kth_32(lane < n ? tmp[lane] : 0u, n, k, lane);
-      small = true;
-    }
-    __syncwarp();
   }
-  if (!small) Ukey = warp_radix_kth(upper_key, Cr, k, hist, lane);
-  const float U = key_float(Ukey);
-  // 6. survivors: lower bound <= U (everything that can still be in the top k)
-  int Cs = 0;
-  for (int base = 0; base < Cr; base += 32) {
-    const int c = base + lane;
-    const bool keep = c < Cr && __fsub_rd(__fmul_rd(cv[c], lo_f), abs32) <= U;
-    const unsigned bal = __ballot_sync(0xffffffffu, keep);
-    const int pos = Cs + __popc(bal & ((1u << lane) - 1));
-    if (keep && pos < kSurvivorCap) si[pos] = ci[c];
-    Cs += __popc(bal);
-  }
-  if (Cs > kSurvivorCap) {
-    if (lane == 0) a.fallback_list[atomicAdd(a.fallback_count, 1)] = (int)(a.row_base + row);
-    return;
-  }
-  __syncwarp();
   // 7. canonical float64 values of the survivors, sort, exact near-tie runs
-  for (int c = lane; c < Cs; c += 32) cs[c] = canonical_d2(q, a.X + (size_t)si[c] * a.d, a.d);
+  // (two interleaved chains a lane when there is more than one round)
+  for (int c = lane; c < Cs; c += 64) {
+    const float* x0 = a.X + (size_t)si[c] * a.d;
+    if (Cs > 32) {
+      const bool two = c + 32 < Cs;
+      double s0, s1;
+      canonical_d2_pair(q, x0, two ? a.X + (size_t)si[c + 32] * a.d : x0, a.d, s0, s1);
+      cs[c] = s0;
+      if (two) cs[c + 32] = s1;
+    } else {
+      cs[c] = canonical_d2(q, x0, a.d);
+    }
+  }
   __syncwarp();
   const unsigned cmp = warp_sort_resolve(cs, si, Cs, k, q, a.X, a.d, lane);
   const int64_t orow = a.perm ? a.perm[row] : row;
@@ -590,16 +732,26 @@ __global__ void __launch_bounds__(kCertWarps * 32, 2)
   certify_row(a, row, smem + (size_t)w * kCertWarpBytes, lane);
 }
 
+// The block's next row for this warp (its previous row's scratch is free).
+__device__ __forceinline__ int claim_row(int* next, int lane) {
+  __syncwarp();
+  return __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(next, 1) : 0, 0);
+}
+
 // Batched form: problem p owns global rows [row_start[p], row_start[p + 1]).
 __global__ void __launch_bounds__(kCertWarps * 32, 2)
     certify_batch_kernel(const CertifyArgs* __restrict__ tab, const int64_t* __restrict__ row_start,
-                         int P, int64_t total) {
+                         int P, int64_t total, int rows) {
   extern __shared__ uint8_t smem[];
+  __shared__ int next;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t r = (int64_t)blockIdx.x * kCertWarps + w;
-  if (r >= total) return;
-  const int p = problem_of(row_start, P, r);
-  certify_row(tab[p], r - row_start[p], smem + (size_t)w * kCertWarpBytes, lane);
+  if (threadIdx.x == 0) next = kCertWarps;
+  __syncthreads();
+  const int64_t row0 = (int64_t)blockIdx.x * rows;
+  for (int i = w; i < rows && row0 + i < total; i = claim_row(&next, lane)) {
+    const int p = problem_of(row_start, P, row0 + i);
+    certify_row(tab[p], row0 + i - row_start[p], smem + (size_t)w * kCertWarpBytes, lane);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -774,8 +926,9 @@ void launch_certify_batch(const CertifyArgs* tab, const int64_t* row_start, int 
   const size_t smem = (size_t)kCertWarps * kCertWarpBytes;
   cudaFuncSetAttribute(certify_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)smem);
-  const unsigned grid = (unsigned)((total_rows + kCertWarps - 1) / kCertWarps);
-  certify_batch_kernel<<<grid, kCertWarps * 32, smem, st>>>(tab, row_start, P, total_rows);
+  const int rows = cert_batch_rows(total_rows);
+  const unsigned grid = (unsigned)((total_rows + rows - 1) / rows);
+  certify_batch_kernel<<<grid, kCertWarps * 32, smem, st>>>(tab, row_start, P, total_rows, rows);
 }
 
 void launch_exact_batch(const ExactArgs* tab, const int64_t* row_start, int P, const int* rows,

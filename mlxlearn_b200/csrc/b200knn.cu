@@ -140,12 +140,14 @@ static int check_device(int device) {
   if (cudaGetDeviceCount(&count) != cudaSuccess || count <= 0)
     return fail(B2K_EUNSUPPORTED, "no CUDA device is available");
   if (device < 0 || device >= count) return fail(B2K_EINVAL, "invalid device %d", device);
-  cudaDeviceProp prop;
-  if (cudaGetDeviceProperties(&prop, device) != cudaSuccess)
-    return fail(B2K_ECUDA, "cudaGetDeviceProperties failed");
-  if (prop.major != 10)
+  // (cudaGetDeviceProperties takes 2.6 ms: more than most of an index's build)
+  int major = 0, minor = 0;
+  if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device) != cudaSuccess)
+    return fail(B2K_ECUDA, "cudaDeviceGetAttribute failed");
+  if (major != 10)
     return fail(B2K_EUNSUPPORTED, "libb200knn needs an sm_100 (B200) device, found sm_%d%d",
-                prop.major, prop.minor);
+                major, minor);
   return B2K_OK;
 }
 
@@ -159,6 +161,27 @@ static int dalloc(T** p, size_t count, cudaStream_t st) {
     return fail(e == cudaErrorMemoryAllocation ? B2K_ENOMEM : B2K_ECUDA,
                 "device allocation of %zu bytes failed: %s", count * sizeof(T),
                 cudaGetErrorString(e));
+  return B2K_OK;
+}
+
+// A buffer of the index (freed with it).  Buffers of up to kPoolAlloc bytes come
+// from the stream-ordered pool: a cudaMalloc or cudaFree costs 40 to 60 us, and
+// an index of a training step lives for one call (17 buffers, 1.8 ms of the 6.5
+// ms of 32,768 x 64 rows against themselves).  Larger ones are given back to the
+// device when freed, so what the pool keeps stays small.  The index's creators
+// synchronise its stream before any other stream sees a buffer.
+constexpr size_t kPoolAlloc = (size_t)32 << 20;
+template <typename T>
+static int ialloc(Index& ix, T** p, size_t count) {
+  const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+  const bool pooled = bytes <= kPoolAlloc;
+  void* v = nullptr;
+  const cudaError_t e = pooled ? cudaMallocAsync(&v, bytes, ix.stream) : cudaMalloc(&v, bytes);
+  if (e != cudaSuccess)
+    return fail(e == cudaErrorMemoryAllocation ? B2K_ENOMEM : B2K_ECUDA,
+                "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+  ix.owned.emplace_back(v, pooled);
+  *p = static_cast<T*>(v);
   return B2K_OK;
 }
 
@@ -213,12 +236,13 @@ static int finish_index(Index& ix, cudaStream_t st) {
 // Pivots for query grouping and row grouping (the caller holds ix.mu).
 static int make_pivots(Index& ix) {
   if (ix.pivots) return B2K_OK;
+  int rc;
   ix.n_pivots = pivot_count(ix.n);
-  B2K_CUDA(cudaMalloc(&ix.pivots, (size_t)ix.n_pivots * ix.d * sizeof(float)));
-  B2K_CUDA(cudaMalloc(&ix.pivot_norms, (size_t)ix.n_pivots * sizeof(float)));
+  if ((rc = ialloc(ix, &ix.pivots, (size_t)ix.n_pivots * ix.d))) return rc;
+  if ((rc = ialloc(ix, &ix.pivot_norms, (size_t)ix.n_pivots))) return rc;
   ix.pivot_dpa = pivot_dims_padded(ix.d);
-  B2K_CUDA(cudaMalloc(&ix.pivots_h,
-                      (size_t)pivot_rows_padded(ix.n_pivots) * ix.pivot_dpa * sizeof(uint16_t)));
+  if ((rc = ialloc(ix, &ix.pivots_h, (size_t)pivot_rows_padded(ix.n_pivots) * ix.pivot_dpa)))
+    return rc;
   launch_pivots(&ix, ix.stream);
   B2K_CUDA(cudaGetLastError());
   B2K_CUDA(cudaStreamSynchronize(ix.stream));
@@ -234,47 +258,27 @@ static bool group_rows_enabled(const Index& ix) {
 }
 
 // Operand row order grouped by nearest pivot (the caller holds ix.mu): a
-// counting sort on the host, stable, so rows keep their training order
-// within a group and the layout is the same on every build.
+// stable counting sort on the device, so rows keep their training order within
+// a group and the layout is the same on every build.
 static int make_row_groups(Index& ix) {
   cudaStream_t st = ix.stream;
   int rc = make_pivots(ix);
   if (rc) return rc;
   const int P = ix.n_pivots;
-  int *key = nullptr, *hist = nullptr;
-  B2K_CUDA(cudaMalloc(&key, (size_t)ix.n * sizeof(int)));
-  if (cudaMalloc(&hist, (size_t)P * sizeof(int)) != cudaSuccess) {
-    cudaFree(key);
-    return fail(B2K_ENOMEM, "device allocation failed");
-  }
+  StreamFree fr{st, {}};
+  int *key = nullptr, *hist = nullptr, *tiles = nullptr;
+  if ((rc = dalloc(&key, (size_t)ix.n, st))) return rc;
+  fr.keep(key);
+  if ((rc = dalloc(&hist, (size_t)P, st))) return rc;
+  fr.keep(hist);
+  if ((rc = dalloc(&tiles, row_group_scratch(ix.n, P), st))) return rc;
+  fr.keep(tiles);
+  if ((rc = ialloc(ix, &ix.xperm, (size_t)ix.n))) return rc;
+  if ((rc = ialloc(ix, &ix.xinv, (size_t)ix.n))) return rc;
+  if ((rc = ialloc(ix, &ix.group_start, (size_t)P + 1))) return rc;
   launch_assign_rows(&ix, ix.X, ix.n, key, hist, st);
-  std::vector<int> hkey((size_t)ix.n);
-  cudaError_t e = cudaMemcpyAsync(hkey.data(), key, (size_t)ix.n * sizeof(int),
-                                  cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaFree(key);
-  cudaFree(hist);
-  if (e != cudaSuccess) return fail(B2K_ECUDA, "row grouping: %s", cudaGetErrorString(e));
-  std::vector<int64_t> start((size_t)P + 1, 0);
-  for (int64_t r = 0; r < ix.n; ++r) ++start[(size_t)hkey[(size_t)r] + 1];
-  for (int p = 0; p < P; ++p) start[(size_t)p + 1] += start[(size_t)p];
-  std::vector<int> gstart(start.begin(), start.end());  // before the scatter advances them
-  std::vector<int> perm((size_t)ix.n), inv((size_t)ix.n);
-  for (int64_t r = 0; r < ix.n; ++r) {
-    const int64_t pos = start[(size_t)hkey[(size_t)r]]++;
-    perm[(size_t)pos] = (int)r;
-    inv[(size_t)r] = (int)pos;
-  }
-  B2K_CUDA(cudaMalloc(&ix.xperm, (size_t)ix.n * sizeof(int)));
-  B2K_CUDA(cudaMalloc(&ix.xinv, (size_t)ix.n * sizeof(int)));
-  B2K_CUDA(cudaMemcpyAsync(ix.xperm, perm.data(), (size_t)ix.n * sizeof(int),
-                           cudaMemcpyHostToDevice, st));
-  B2K_CUDA(cudaMemcpyAsync(ix.xinv, inv.data(), (size_t)ix.n * sizeof(int),
-                           cudaMemcpyHostToDevice, st));
-  B2K_CUDA(cudaMalloc(&ix.group_start, gstart.size() * sizeof(int)));
-  B2K_CUDA(cudaMemcpyAsync(ix.group_start, gstart.data(), gstart.size() * sizeof(int),
-                           cudaMemcpyHostToDevice, st));
-  B2K_CUDA(cudaStreamSynchronize(st));
+  launch_row_groups(key, ix.n, P, hist, tiles, ix.group_start, ix.xperm, ix.xinv, st);
+  B2K_CUDA(cudaGetLastError());
   return B2K_OK;
 }
 
@@ -301,7 +305,7 @@ static int ensure_bf16(Index& ix) {
   ix.n_pad_tc = round_up(ix.n, kTcBN);
   int rc;
   if ((rc = ensure_row_groups(ix))) return rc;
-  B2K_CUDA(cudaMalloc(&ix.Xh, (size_t)ix.n_pad_tc * ix.dp * sizeof(uint16_t)));
+  if ((rc = ialloc(ix, &ix.Xh, (size_t)ix.n_pad_tc * ix.dp))) return rc;
   launch_prep_index_bf16(&ix, ix.Xh, st, ix.xperm);
   B2K_CUDA(cudaGetLastError());
   float stats[kStatsLen];
@@ -311,8 +315,8 @@ static int ensure_bf16(Index& ix) {
   if (!tensor_map_2d_bf16(&ix.tmap_b, ix.Xh, (uint64_t)ix.dp, (uint64_t)ix.n_pad_tc, kTcBK, kTcBN))
     return fail(B2K_ECUDA, "cuTensorMapEncodeTiled failed for the reference rows");
   // norm columns of the reference rows and the matching query-side ones
-  B2K_CUDA(cudaMalloc(&ix.Xaug, (size_t)ix.n_pad_tc * kTcAug * sizeof(uint16_t)));
-  B2K_CUDA(cudaMalloc(&ix.aug_ones, (size_t)kTcBM * kTcAug * sizeof(uint16_t)));
+  if ((rc = ialloc(ix, &ix.Xaug, (size_t)ix.n_pad_tc * kTcAug))) return rc;
+  if ((rc = ialloc(ix, &ix.aug_ones, (size_t)kTcBM * kTcAug))) return rc;
   launch_prep_aug(&ix, ix.Xaug, ix.aug_ones, st, ix.xperm);
   B2K_CUDA(cudaGetLastError());
   B2K_CUDA(cudaStreamSynchronize(st));
@@ -333,11 +337,11 @@ static int ensure_tf32(Index& ix) {
   ix.n_pad_tc = round_up(ix.n, kTcBN);
   int rc;
   if ((rc = ensure_row_groups(ix))) return rc;
-  B2K_CUDA(cudaMalloc(&ix.Xt, (size_t)ix.n_pad_tc * ix.dpt * sizeof(float)));
+  if ((rc = ialloc(ix, &ix.Xt, (size_t)ix.n_pad_tc * ix.dpt))) return rc;
   launch_prep_index_tf32(&ix, ix.Xt, st, ix.xperm);
   B2K_CUDA(cudaGetLastError());
-  B2K_CUDA(cudaMalloc(&ix.Xtaug, (size_t)ix.n_pad_tc * kTcAugF * sizeof(float)));
-  B2K_CUDA(cudaMalloc(&ix.taug_ones, (size_t)kTcBM * kTcAugF * sizeof(float)));
+  if ((rc = ialloc(ix, &ix.Xtaug, (size_t)ix.n_pad_tc * kTcAugF))) return rc;
+  if ((rc = ialloc(ix, &ix.taug_ones, (size_t)kTcBM * kTcAugF))) return rc;
   launch_prep_aug_tf32(&ix, ix.Xtaug, ix.taug_ones, st, ix.xperm);
   B2K_CUDA(cudaGetLastError());
   float stats[kStatsLen];
@@ -961,18 +965,24 @@ static int build_from_device(b2k_index* h, const float* src, cudaMemcpyKind kind
   keep_pool(ix.device);
   B2K_CUDA(cudaStreamCreateWithFlags(&ix.stream, cudaStreamNonBlocking));
   const size_t bytes = (size_t)ix.n * ix.d * sizeof(float);
-  B2K_CUDA(cudaMalloc(&ix.X, bytes));
-  B2K_CUDA(cudaMalloc(&ix.nx32, (size_t)ix.n * sizeof(float)));
-  B2K_CUDA(cudaMalloc(&ix.center, (size_t)ix.d * sizeof(float)));
-  B2K_CUDA(cudaMalloc(&ix.colsum, (size_t)ix.d * sizeof(double)));
-  B2K_CUDA(cudaMalloc(&ix.nx64, (size_t)ix.n * sizeof(double)));
-  B2K_CUDA(cudaMalloc(&ix.stats_dev, kStatsLen * sizeof(float)));
-  if (kind == cudaMemcpyDeviceToDevice && user_st) {
-    B2K_CUDA(cudaMemcpyAsync(ix.X, src, bytes, kind, user_st));
-    B2K_CUDA(cudaStreamSynchronize(user_st));
-  } else {
-    B2K_CUDA(cudaMemcpyAsync(ix.X, src, bytes, kind, ix.stream));
+  int rc;
+  if ((rc = ialloc(ix, &ix.X, (size_t)ix.n * ix.d))) return rc;
+  if ((rc = ialloc(ix, &ix.nx32, (size_t)ix.n))) return rc;
+  if ((rc = ialloc(ix, &ix.center, (size_t)ix.d))) return rc;
+  if ((rc = ialloc(ix, &ix.colsum, (size_t)ix.d))) return rc;
+  if ((rc = ialloc(ix, &ix.nx64, (size_t)ix.n))) return rc;
+  if ((rc = ialloc(ix, &ix.stats_dev, kStatsLen))) return rc;
+  if (kind == cudaMemcpyDeviceToDevice) {
+    // after the caller's work on its stream (NULL: the legacy default stream),
+    // which the index's own stream does not wait for by itself
+    cudaEvent_t ready;
+    B2K_CUDA(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+    cudaError_t e = cudaEventRecord(ready, user_st);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(ix.stream, ready, 0);
+    cudaEventDestroy(ready);
+    B2K_CUDA(e);
   }
+  B2K_CUDA(cudaMemcpyAsync(ix.X, src, bytes, kind, ix.stream));
   return finish_index(ix, ix.stream);
 }
 
@@ -1026,24 +1036,14 @@ int b2k_index_destroy(b2k_index* h) {
   Index& ix = h->ix;
   cudaSetDevice(ix.device);
   if (ix.stream) cudaStreamSynchronize(ix.stream);
-  cudaFree(ix.X);
-  cudaFree(ix.nx32);
-  cudaFree(ix.center);
-  cudaFree(ix.colsum);
-  cudaFree(ix.nx64);
-  cudaFree(ix.stats_dev);
-  cudaFree(ix.Xh);
-  cudaFree(ix.pivots);
-  cudaFree(ix.pivot_norms);
-  cudaFree(ix.pivots_h);
-  cudaFree(ix.Xaug);
-  cudaFree(ix.aug_ones);
-  cudaFree(ix.xperm);
-  cudaFree(ix.xinv);
-  cudaFree(ix.group_start);
-  cudaFree(ix.Xt);
-  cudaFree(ix.Xtaug);
-  cudaFree(ix.taug_ones);
+  // work on other streams may still read the index: as cudaFree would, wait
+  cudaDeviceSynchronize();
+  for (auto& b : ix.owned) {
+    if (b.second)
+      cudaFreeAsync(b.first, ix.stream);
+    else
+      cudaFree(b.first);
+  }
   cudaFree(ix.Xu);
   cudaFree(ix.nxu);
   if (ix.stream) cudaStreamDestroy(ix.stream);

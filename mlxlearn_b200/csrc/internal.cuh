@@ -5,6 +5,8 @@
 
 #include <cstdint>
 #include <mutex>
+#include <utility>
+#include <vector>
 
 #include "../../include/b200knn.h"
 
@@ -123,6 +125,9 @@ struct Index {
   uint16_t* pivots_h = nullptr;  // bf16 pivots for the assignment, zero padded:
   int pivot_dpa = 0;             // [pivot_rows_padded(n_pivots), pivot_dpa]
   cudaStream_t stream = nullptr;
+  // every buffer above but the u8 ones, and whether it came from the
+  // stream-ordered pool
+  std::vector<std::pair<void*, bool>> owned;
   std::mutex mu;
 };
 
@@ -230,6 +235,12 @@ void launch_query_order(const Index* ix, const float* Q, int64_t m, int* key, in
 // hist[p] = rows per pivot
 void launch_assign_rows(const Index* ix, const float* X, int64_t n, int* key, int* hist,
                         cudaStream_t st);
+// Rows grouped by key, stable: group_start[P + 1], perm (group position -> row)
+// and inv (its inverse).  hist[p] = rows of key p; tiles holds
+// row_group_scratch(n, P) ints.
+size_t row_group_scratch(int64_t n, int P);
+void launch_row_groups(const int* key, int64_t n, int P, const int* hist, int* tiles,
+                       int* group_start, int* perm, int* inv, cudaStream_t st);
 // home[t] = first reference tile of query tile t's window of `window` tiles:
 // the tiles holding the grouped rows of the pivot nearest to the tile's
 // middle query (perm, key: the query order and pivot keys of

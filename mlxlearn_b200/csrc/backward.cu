@@ -17,6 +17,8 @@
 // point-set losses such as a Chamfer term.
 #include <cuda_runtime.h>
 
+#include <climits>
+
 #include "common.cuh"
 #include "internal.cuh"
 
@@ -204,36 +206,131 @@ __global__ void grad_x_narrow_kernel(const float* __restrict__ Q, const float* _
     if (f < d) dX[r * d + f] = acc[f];
 }
 
-// One warp per reference row: put its bucket in ascending flat position
-// (each lane ranks some entries against the whole bucket and writes them to
-// `sorted`: linear per entry, so rows that many queries picked stay cheap),
-// then accumulate in that order.
+// Wide rows: every bucket is put in ascending flat position (each entry ranks
+// itself against the bucket; positions are distinct) and summed in that order.
+// One warp a reference row up to kBigBucket entries.  Larger buckets (rows that
+// many queries picked: on 32,768 x 64 N(0, 1) rows, k = 8, the largest hold
+// over a thousand) are listed for one block each: ranking costs the square of
+// the bucket, and a warp walking it one dependent load at a time kept a few
+// warps busy for 0.48 ms while the other rows took 0.05.
+constexpr int kBigBucket = 128;
+constexpr int kBigThreads = 256;
+constexpr int kBigStage = 2048;  // entries staged in shared memory at a time
+
 __global__ void grad_x_kernel(const float* __restrict__ Q, const float* __restrict__ X,
                               const float* __restrict__ G, const float* __restrict__ E,
                               const int* __restrict__ offsets, const int* __restrict__ order,
                               int* __restrict__ sorted, int64_t n, int d, int k, int squared,
+                              int* __restrict__ big, int* __restrict__ big_count,
                               float* __restrict__ dX) {
   const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (r >= n) return;
   const int a = offsets[r], b = offsets[r + 1], cnt = b - a;
-  for (int e = lane; e < cnt; e += 32) {
-    const int v = order[a + e];
+  if (cnt > kBigBucket) {
+    if (lane == 0) big[atomicAdd(big_count, 1)] = (int)r;
+    return;
+  }
+  for (int e0 = 0; e0 < cnt; e0 += 32) {
+    const int v = e0 + lane < cnt ? order[a + e0 + lane] : INT_MAX;
     int rank = 0;
-    for (int f = 0; f < cnt; ++f) rank += order[a + f] < v;  // flat positions are distinct
-    sorted[a + rank] = v;
+    for (int f0 = 0; f0 < cnt; f0 += 32) {
+      const int u = f0 + lane < cnt ? order[a + f0 + lane] : INT_MAX;
+#pragma unroll 8
+      for (int l = 0; l < 32; ++l) rank += __shfl_sync(0xffffffffu, u, l) < v;
+    }
+    if (e0 + lane < cnt) sorted[a + rank] = v;
   }
   __syncwarp();
-  for (int f = lane; f < d; f += 32) {
-    const float x = X[r * d + f];
+  for (int f0 = 0; f0 < d; f0 += 32) {
+    const int f = f0 + lane;
+    const float x = f < d ? X[r * d + f] : 0.0f;
     float acc = 0.0f;
-    for (int p = a; p < b; ++p) {
-      const int t = sorted[p];
-      const int64_t i = t / k;
-      const float c = coef_of(G[t], E ? E[t] : 0.0f, squared);
-      acc = fmaf(c, x - Q[i * d + f], acc);
+    for (int p0 = 0; p0 < cnt; p0 += 32) {
+      // the lanes fetch 32 entries together; the sum takes them in order, four
+      // query rows in flight
+      int64_t my_i = 0;
+      float my_c = 0.0f;
+      if (p0 + lane < cnt) {
+        const int t = sorted[a + p0 + lane];
+        my_i = t / k;
+        my_c = coef_of(G[t], E ? E[t] : 0.0f, squared);
+      }
+      const int stop = min(32, cnt - p0);
+      for (int l = 0; l < stop; l += 4) {
+        float q[4], c[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int64_t i = __shfl_sync(0xffffffffu, my_i, l + u);
+          c[u] = __shfl_sync(0xffffffffu, my_c, l + u);
+          q[u] = (l + u < stop && f < d) ? Q[i * d + f] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (l + u < stop) acc = fmaf(c[u], x - q[u], acc);
+      }
     }
-    dX[r * d + f] = acc;
+    if (f < d) dX[r * d + f] = acc;
+  }
+}
+
+// One block a listed row (a fixed grid walks the list).
+__global__ void __launch_bounds__(kBigThreads)
+    grad_x_big_kernel(const float* __restrict__ Q, const float* __restrict__ X,
+                      const float* __restrict__ G, const float* __restrict__ E,
+                      const int* __restrict__ offsets, const int* __restrict__ order,
+                      int* __restrict__ sorted, int d, int k, int squared,
+                      const int* __restrict__ big, const int* __restrict__ big_count,
+                      float* __restrict__ dX) {
+  __shared__ int s_key[kBigStage];
+  __shared__ float s_c[kBigStage];
+  const int listed = *big_count;
+  for (int w = blockIdx.x; w < listed; w += gridDim.x) {
+    const int64_t r = big[w];
+    const int a = offsets[r], cnt = offsets[r + 1] - a;
+    for (int e0 = 0; e0 < cnt; e0 += kBigThreads) {
+      const int e = e0 + threadIdx.x;
+      const int v = e < cnt ? order[a + e] : INT_MAX;
+      int rank = 0;
+      for (int f0 = 0; f0 < cnt; f0 += kBigStage) {
+        const int len = min(kBigStage, cnt - f0);
+        __syncthreads();
+        for (int f = threadIdx.x; f < len; f += kBigThreads) s_key[f] = order[a + f0 + f];
+        __syncthreads();
+#pragma unroll 8
+        for (int f = 0; f < len; ++f) rank += s_key[f] < v;
+      }
+      if (e < cnt) sorted[a + rank] = v;
+    }
+    __syncthreads();  // the block's writes to `sorted`
+    for (int g0 = 0; g0 < d; g0 += kBigThreads) {
+      const int f = g0 + threadIdx.x;
+      const float x = f < d ? X[r * d + f] : 0.0f;
+      float acc = 0.0f;
+      for (int p0 = 0; p0 < cnt; p0 += kBigStage) {
+        const int len = min(kBigStage, cnt - p0);
+        __syncthreads();
+        for (int p = threadIdx.x; p < len; p += kBigThreads) {
+          const int t = sorted[a + p0 + p];
+          s_key[p] = t / k;
+          s_c[p] = coef_of(G[t], E ? E[t] : 0.0f, squared);
+        }
+        __syncthreads();
+        if (f < d) {
+          int p = 0;
+          for (; p + 8 <= len; p += 8) {  // eight query rows in flight, summed in order
+            float q[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) q[u] = Q[(int64_t)s_key[p + u] * d + f];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) acc = fmaf(s_c[p + u], x - q[u], acc);
+          }
+          for (; p < len; ++p) acc = fmaf(s_c[p], x - Q[(int64_t)s_key[p] * d + f], acc);
+        }
+      }
+      if (f < d) dX[r * d + f] = acc;
+    }
+    __syncthreads();  // before the next row's staging
   }
 }
 
@@ -274,9 +371,18 @@ int knn_backward(const float* Q, int64_t m, const float* X, int64_t n, int d, in
     if (narrow)
       grad_x_narrow_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
           Q, X, G, E, offsets, order, n, d, k, squared, dX);
-    else
+    else {
+      // the bucket cursors and counts are free by now: the big rows and their number
+      int* big = cursor;
+      int* big_count = counts;
+      cudaMemsetAsync(big_count, 0, sizeof(int), st);
       grad_x_kernel<<<(unsigned)((n + warps - 1) / warps), warps * 32, 0, st>>>(
-          Q, X, G, E, offsets, order, sorted, n, d, k, squared, dX);
+          Q, X, G, E, offsets, order, sorted, n, d, k, squared, big, big_count, dX);
+      int dev = 0;
+      cudaGetDevice(&dev);
+      grad_x_big_kernel<<<4 * num_sms(dev), kBigThreads, 0, st>>>(
+          Q, X, G, E, offsets, order, sorted, d, k, squared, big, big_count, dX);
+    }
   }
   return (int)cudaGetLastError();
 }

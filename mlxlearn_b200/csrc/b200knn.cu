@@ -17,7 +17,10 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -81,6 +84,20 @@ int num_sms(int device) {
     cached[device] = v;
   }
   return cached[device];
+}
+
+cudaError_t allow_smem_impl(const void* kernel, size_t bytes) {
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  static std::mutex mu;
+  static std::map<std::pair<const void*, int>, size_t> limits;  // one entry per kernel and device
+  std::lock_guard<std::mutex> lock(mu);
+  size_t& limit = limits[{kernel, device}];
+  if (limit >= bytes) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) limit = bytes;
+  return e;
 }
 
 // --------------------------------------------------------------- TMA maps
@@ -215,6 +232,40 @@ struct StreamFree {
     ptrs.push_back(p);
     return p;
   }
+};
+
+// The scratch of one call as one stream-ordered allocation: buffers are reserved
+// first (256-byte aligned), then placed.  Seventeen cudaMallocAsync and as many
+// frees, four memsets and three reads back were 70 of the 155 us of a 2,000
+// query call.
+class Workspace {
+ public:
+  template <typename T>
+  void reserve(T** p, size_t count) {
+    slots_.push_back({reinterpret_cast<void**>(p), bytes_});
+    bytes_ += (std::max<size_t>(count, 1) * sizeof(T) + 255) / 256 * 256;
+  }
+  size_t bytes() const { return bytes_; }
+  int place(cudaStream_t st, StreamFree& fr) {
+    unsigned char* base = nullptr;
+    const int rc = dalloc(&base, bytes_, st);
+    if (rc) return rc;
+    fr.keep(base);
+    for (auto& s : slots_) *s.first = base + s.second;
+    return B2K_OK;
+  }
+
+ private:
+  std::vector<std::pair<void**, size_t>> slots_;
+  size_t bytes_ = 0;
+};
+
+// Error word, counts and flags of a kNN call, zeroed together and read back
+// together.
+struct CallState {
+  int status[8];                     // [0] error, [2] uncertified rows, [4] range, [5] nonfinite,
+                                     // [6] [7] claimed units of the screens
+  unsigned long long counters[8];
 };
 
 static int finish_index(Index& ix, cudaStream_t st) {
@@ -604,29 +655,31 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
     for (auto& e : ev) cudaEventCreate(&e);
   if (stats) cudaEventRecord(ev[0], st);
 
-  int* status = nullptr;
-  unsigned long long* counters = nullptr;
-  if ((rc = dalloc(&status, 8, st))) return rc;
-  fr.keep(status);
-  if ((rc = dalloc(&counters, 8, st))) return rc;
-  fr.keep(counters);
-  B2K_CUDA(cudaMemsetAsync(status, 0, 8 * sizeof(int), st));
-  B2K_CUDA(cudaMemsetAsync(counters, 0, 8 * sizeof(unsigned long long), st));
-  // NaN / inf queries: flagged on the device, reported with the final status
-  // read (the search itself stays bounded on such inputs)
-  launch_nonfinite_check(dQ, m * (int64_t)ix.d, status + 5, st);
-
   int S = 1;
   int64_t second_pass_rows = 0, second_exact_rows = 0;
-  if (mode == B2K_MODE_EXACT) {
-    rc = run_exact(ix, dQ, m, k, exclude_self, q_offset, d_dist, d_idx, nullptr, nullptr,
-                   counters, status, st, fr, true, ext_perm, squared);
-    if (rc) return rc;
-  } else if (mode == B2K_MODE_U8) {
-    if (stats) cudaEventRecord(ev[1], st);
-    rc = run_u8(ix, dQ, m, k, exclude_self, q_offset, d_dist, d_idx, squared, status, st, fr, &S);
-    if (rc) return rc;
-    if (stats) cudaEventRecord(ev[2], st);
+  CallState* state = nullptr;
+  CallState h;
+  if (mode == B2K_MODE_EXACT || mode == B2K_MODE_U8) {
+    if ((rc = dalloc(&state, 1, st))) return rc;
+    fr.keep(state);
+    B2K_CUDA(cudaMemsetAsync(state, 0, sizeof(CallState), st));
+    // NaN / inf queries: flagged on the device, reported with the final state
+    // (the search itself stays bounded on such inputs)
+    launch_nonfinite_check(dQ, m * (int64_t)ix.d, state->status + 5, st);
+    if (mode == B2K_MODE_EXACT) {
+      rc = run_exact(ix, dQ, m, k, exclude_self, q_offset, d_dist, d_idx, nullptr, nullptr,
+                     state->counters, state->status, st, fr, true, ext_perm, squared);
+      if (rc) return rc;
+    } else {
+      if (stats) cudaEventRecord(ev[1], st);
+      rc = run_u8(ix, dQ, m, k, exclude_self, q_offset, d_dist, d_idx, squared, state->status, st,
+                  fr, &S);
+      if (rc) return rc;
+      if (stats) cudaEventRecord(ev[2], st);
+    }
+    if (stats) cudaEventRecord(ev[3], st);
+    B2K_CUDA(cudaMemcpyAsync(&h, state, sizeof(h), cudaMemcpyDeviceToHost, st));
+    B2K_CUDA(cudaStreamSynchronize(st));
   } else {
     if (mode == B2K_MODE_BF16 && (rc = ensure_bf16(ix))) return rc;
     if (mode == B2K_MODE_TF32 && (rc = ensure_tf32(ix))) return rc;
@@ -637,63 +690,70 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
     const int64_t n_tiles = tc ? ix.n_pad_tc / kTcBN : (ix.n + kSimtBN - 1) / kSimtBN;
     const int sms = num_sms(ix.device);
     S = choose_splits(m_pad / bm, n_tiles, tc ? sms : 2 * sms);
+    const bool lazy = tc && tc_lazy_sink(k);  // its screen leaves V_k to the lists
     // lists per query: one per (split, column group of the screen)
     const int S_lists = S * (tc ? tc_column_groups(k) : simt_column_groups(kSinkKnn));
     // Group nearby queries (reorder.cu); results go back to the original rows.
+    const bool grouped = !ext_perm && m >= 2048 && reorder_enabled();
+    if (grouped && (rc = ensure_pivots(ix))) return rc;
+    const int64_t m_tiles = m_pad / kTcBM;
+    const int kSeedTiles = seed_tiles();
+    const bool seed = tc && grouped && ix.group_start && n_tiles >= 2 * kSeedTiles &&
+                      seed_enabled();
+    const int seed_k = lazy ? 16 : k, seed_groups = tc ? tc_column_groups(seed_k) : 0;
+
+    Workspace ws;
+    int *hist = nullptr, *key = nullptr, *pm = nullptr, *home = nullptr, *seed_counts = nullptr;
+    float *Qp = nullptr, *seed_kth = nullptr;
+    uint32_t* shared_kth = nullptr;
+    int* fb_list = nullptr;
+    QueryPrep qp{};
+    ScreenOut so{};
+    // zeroed: the call's state and the pivot histogram of the query order
+    ws.reserve(&state, 1);
+    if (grouped) ws.reserve(&hist, (size_t)ix.n_pivots);
+    const size_t zeroed = ws.bytes();
+    if (grouped) {
+      ws.reserve(&key, (size_t)m);  // nearest pivot of each query
+      ws.reserve(&pm, (size_t)m);
+      ws.reserve(&Qp, (size_t)m * ix.d);
+    }
+    ws.reserve(&shared_kth, (size_t)m_pad);
+    ws.reserve(&qp.E, (size_t)m_pad);
+    ws.reserve(&qp.nq, (size_t)m_pad);  // ||y_q||^2 for certify's two-stage refinement
+    if (tc && !tf32) ws.reserve(&qp.Ah, (size_t)m_pad * ix.dp);
+    if (tf32) ws.reserve(&qp.At, (size_t)m_pad * ix.dpt);
+    // the register trackers' lists hold 4 x kListCap entries per (split, query)
+    // whatever the column groups (the lazy tracker's select is sized for kListCap)
+    so.cap = (tc && !lazy) ? kListCap * 4 / tc_column_groups(k) : kListCap;
+    so.m_pad = (int)m_pad;
+    ws.reserve(&so.lists, (size_t)S_lists * m_pad * so.cap);
+    ws.reserve(&so.counts, (size_t)S_lists * m_pad);
+    if (!lazy) ws.reserve(&so.kth, (size_t)S_lists * m_pad * k);
+    if (seed) {
+      ws.reserve(&home, (size_t)m_tiles);
+      ws.reserve(&seed_counts, (size_t)seed_groups * m_pad);
+      ws.reserve(&seed_kth, (size_t)seed_groups * m_pad * seed_k);
+    }
+    ws.reserve(&fb_list, (size_t)m);
+    if ((rc = ws.place(st, fr))) return rc;
+    int* status = state->status;
+    unsigned long long* counters = state->counters;
+    B2K_CUDA(cudaMemsetAsync(state, 0, zeroed, st));
+
     const int* perm = ext_perm;
     const float* Qs = dQ;
-    int* key = nullptr;  // nearest pivot of each query (query grouping)
-    if (!ext_perm && m >= 2048 && reorder_enabled()) {
-      if ((rc = ensure_pivots(ix))) return rc;
-      int *hist = nullptr, *pm = nullptr;
-      float* Qp = nullptr;
-      if ((rc = dalloc(&key, (size_t)m, st))) return rc;
-      fr.keep(key);
-      if ((rc = dalloc(&hist, (size_t)ix.n_pivots, st))) return rc;
-      fr.keep(hist);
-      if ((rc = dalloc(&pm, (size_t)m, st))) return rc;
-      fr.keep(pm);
-      if ((rc = dalloc(&Qp, (size_t)m * ix.d, st))) return rc;
-      fr.keep(Qp);
+    if (grouped) {
       launch_query_order(&ix, dQ, m, key, hist, pm, Qp, st);
       B2K_CUDA(cudaGetLastError());
       perm = pm;
       Qs = Qp;
     }
-    uint32_t* shared_kth = nullptr;
-    if ((rc = dalloc(&shared_kth, (size_t)m_pad, st))) return rc;
-    fr.keep(shared_kth);
-    B2K_CUDA(cudaMemsetAsync(shared_kth, 0xff, (size_t)m_pad * sizeof(uint32_t), st));
-    QueryPrep qp{};
-    if ((rc = dalloc(&qp.E, (size_t)m_pad, st))) return rc;
-    fr.keep(qp.E);
-    qp.flags = status + 4;  // shares the zeroed status block
-    // ||y_q||^2 for the certify pass's two-stage refinement
-    if ((rc = dalloc(&qp.nq, (size_t)m_pad, st))) return rc;
-    fr.keep(qp.nq);
-    if (tc && !tf32) {
-      if ((rc = dalloc(&qp.Ah, (size_t)m_pad * ix.dp, st))) return rc;
-      fr.keep(qp.Ah);
-    }
-    if (tf32) {
-      if ((rc = dalloc(&qp.At, (size_t)m_pad * ix.dpt, st))) return rc;
-      fr.keep(qp.At);
-    }
+    qp.flags = status + 4;
+    qp.nonfinite = status + 5;  // NaN / inf queries, reported with the final state
+    qp.shared_kth = shared_kth;
     launch_prep_queries(&ix, Qs, m, m_pad, mode, qp, st);
     B2K_CUDA(cudaGetLastError());
-    ScreenOut so{};
-    // the register trackers' lists hold 4 x kListCap entries per (split, query)
-    // whatever the column groups (the lazy tracker's select is sized for kListCap)
-    so.cap = (tc && !tc_lazy_sink(k)) ? kListCap * 4 / tc_column_groups(k) : kListCap;
-    so.m_pad = (int)m_pad;
-    if ((rc = dalloc(&so.lists, (size_t)S_lists * m_pad * so.cap, st))) return rc;
-    fr.keep(so.lists);
-    if ((rc = dalloc(&so.counts, (size_t)S_lists * m_pad, st))) return rc;
-    fr.keep(so.counts);
-    if (!(tc && tc_lazy_sink(k))) {  // lazy screens leave V_k to the lists
-      if ((rc = dalloc(&so.kth, (size_t)S_lists * m_pad * k, st))) return rc;
-      fr.keep(so.kth);
-    }
     SinkArgs sa{};
     sa.out = so;
     sa.k = k;
@@ -715,8 +775,6 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
       // capacity 0) to the per-query words the main screen's lists start
       // from.  A published value is the k-th smallest of real screen values
       // of the query, so it is >= the final V_k and the certificate holds.
-      const int64_t m_tiles = m_pad / kTcBM;
-      const int kSeedTiles = seed_tiles();
       //
       // For k > 16 the pass runs the register tracker at its widest, 16 values
       // in each of four column groups, and launch_seed_kth takes the k-th
@@ -725,26 +783,14 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
       // k = 50: list entries 88M -> 37M, screen 5.71 -> 2.38 ms (1.79 with
       // sixteen epilogue warps).  Filling the lazy tracker's own lists in the
       // pass instead cost 2.3 ms, the pass itself 0.45.
-      const bool lazy = tc_lazy_sink(k);
-      if (key && ix.group_start && n_tiles >= 2 * kSeedTiles && seed_enabled()) {
-        const int ks = lazy ? 16 : k;
-        const int G = tc_column_groups(ks);
-        int* home = nullptr;
-        int* seed_counts = nullptr;
-        float* seed_kth = nullptr;
-        if ((rc = dalloc(&home, (size_t)m_tiles, st))) return rc;
-        fr.keep(home);
-        if ((rc = dalloc(&seed_counts, (size_t)G * m_pad, st))) return rc;
-        fr.keep(seed_counts);
-        if ((rc = dalloc(&seed_kth, (size_t)G * m_pad * ks, st))) return rc;
-        fr.keep(seed_kth);
+      if (seed) {
         launch_home_tiles(perm, key, m, ix.group_start, (int)n_tiles, kSeedTiles, home,
                           (int)m_tiles, st);
         SinkArgs sb = sa;
         sb.out.cap = 0;  // the trackers only: no list entry is written
         sb.out.counts = seed_counts;
         sb.out.kth = seed_kth;
-        sb.k = ks;
+        sb.k = seed_k;
         if (lazy) sb.shared_kth = nullptr;  // a group's 16th value is not the query's k-th
         // status[7] (zeroed above) counts this pass's claimed units
         int lr = launch_screen_tc(&ix, &tmap_a, m, m_pad, exclude_self, q_offset, 1, qp.E,
@@ -752,7 +798,8 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
                                   kSeedTiles);
         if (lr) return fail(B2K_ECUDA, "tcgen05 seeding screen launch failed: %s",
                             cudaGetErrorString((cudaError_t)lr));
-        if (lazy && G * ks >= k) launch_seed_kth(seed_kth, G, ks, m, m_pad, k, shared_kth, st);
+        if (lazy && seed_groups * seed_k >= k)
+          launch_seed_kth(seed_kth, seed_groups, seed_k, m, m_pad, k, shared_kth, st);
         if (stats) cudaEventRecord(ev[4], st);
         seeded = true;
       }
@@ -767,9 +814,6 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
       B2K_CUDA(cudaGetLastError());
     }
     if (stats) cudaEventRecord(ev[2], st);
-    int* fb_list = nullptr;
-    if ((rc = dalloc(&fb_list, (size_t)m, st))) return rc;
-    fr.keep(fb_list);
     CertifyArgs ca{};
     ca.X = ix.X;
     ca.Q = Qs;
@@ -798,50 +842,46 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
     // candidates or survivors).  After a bf16 pass they get a second pass with
     // the fp32 screen, whose bound is ~50x tighter; otherwise (and for rows the
     // fp32 pass cannot certify) the exhaustive exact scan.
-    bool second_pass = false;
-    if (tc) {
-      int nfb = 0;
-      B2K_CUDA(cudaMemcpyAsync(&nfb, status + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
-      B2K_CUDA(cudaStreamSynchronize(st));
-      if (nfb > 0) {
-        float* Qfb = nullptr;
-        int* pfb = nullptr;
-        if ((rc = dalloc(&Qfb, (size_t)nfb * ix.d, st))) return rc;
-        fr.keep(Qfb);
-        if ((rc = dalloc(&pfb, (size_t)nfb, st))) return rc;
-        fr.keep(pfb);
-        launch_gather_fallback(Qs, ix.d, fb_list, perm, nfb, Qfb, pfb, st);
-        B2K_CUDA(cudaGetLastError());
-        b2k_stats sub{};
-        rc = knn_device_impl(ix, Qfb, nfb, k, exclude_self, q_offset, B2K_MODE_FP32 | sq_flag,
-                             d_dist, d_idx, st, &sub, pfb);
-        if (rc) return rc;
-        second_pass_rows = nfb;
-        second_exact_rows = sub.fallback_rows;
-      }
-      second_pass = true;
-    }
-    if (!second_pass) {
+    if (!tc) {
       rc = run_exact(ix, Qs, m, k, exclude_self, q_offset, d_dist, d_idx, fb_list, status + 2,
                      counters, status, st, fr, false, perm, squared);
       if (rc) return rc;
     }
+    if (stats) cudaEventRecord(ev[3], st);
+    B2K_CUDA(cudaMemcpyAsync(&h, state, sizeof(h), cudaMemcpyDeviceToHost, st));
+    B2K_CUDA(cudaStreamSynchronize(st));
+    const int nfb = h.status[2];
+    if (tc && nfb > 0 && h.status[0] == DEV_OK && !h.status[5] && !(h.status[4] & 1)) {
+      float* Qfb = nullptr;
+      int* pfb = nullptr;
+      if ((rc = dalloc(&Qfb, (size_t)nfb * ix.d, st))) return rc;
+      fr.keep(Qfb);
+      if ((rc = dalloc(&pfb, (size_t)nfb, st))) return rc;
+      fr.keep(pfb);
+      launch_gather_fallback(Qs, ix.d, fb_list, perm, nfb, Qfb, pfb, st);
+      B2K_CUDA(cudaGetLastError());
+      b2k_stats sub{};
+      rc = knn_device_impl(ix, Qfb, nfb, k, exclude_self, q_offset, B2K_MODE_FP32 | sq_flag,
+                           d_dist, d_idx, st, &sub, pfb);
+      if (rc) return rc;
+      second_pass_rows = nfb;
+      second_exact_rows = sub.fallback_rows;
+      if (stats) {
+        cudaEventRecord(ev[3], st);
+        cudaEventSynchronize(ev[3]);
+      }
+    }
   }
-  if (stats) cudaEventRecord(ev[3], st);
-  int hstatus[8];
-  unsigned long long hcnt[5];
-  B2K_CUDA(cudaMemcpyAsync(hstatus, status, sizeof(hstatus), cudaMemcpyDeviceToHost, st));
-  B2K_CUDA(cudaMemcpyAsync(hcnt, counters, sizeof(hcnt), cudaMemcpyDeviceToHost, st));
-  B2K_CUDA(cudaStreamSynchronize(st));
-  if (fm == 3) hstatus[0] = DEV_TIMEOUT_FULL;
+  const int* hstatus = h.status;
+  const unsigned long long* hcnt = h.counters;
+  const int err = fm == 3 ? (int)DEV_TIMEOUT_FULL : hstatus[0];
   if (hstatus[5]) return fail(B2K_ENONFINITE, "training and query coordinates must be finite");
-  if (hstatus[0] == DEV_TOO_MANY_TIES)
+  if (err == DEV_TOO_MANY_TIES)
     return fail(B2K_EUNSUPPORTED,
                 "more than %d training rows tie (within float64 error) with a query's k-th "
                 "neighbour",
                 kExactCap);
-  if (hstatus[0] != DEV_OK)
-    return fail(B2K_ETIMEOUT, "a bounded device wait gave up (code %d)", hstatus[0]);
+  if (err != DEV_OK) return fail(B2K_ETIMEOUT, "a bounded device wait gave up (code %d)", err);
   if (hstatus[4] & 1) {
     // Some query coordinate is outside the screens' safe range: redo exactly.
     return knn_device_impl(ix, dQ, m, k, exclude_self, q_offset, B2K_MODE_EXACT | sq_flag,

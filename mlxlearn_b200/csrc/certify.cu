@@ -915,7 +915,7 @@ __global__ void __launch_bounds__(kExactThreads)
 void launch_certify(const CertifyArgs& a, cudaStream_t st) {
   if (a.m <= 0) return;
   const size_t smem = (size_t)kCertWarps * kCertWarpBytes;
-  cudaFuncSetAttribute(certify_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(certify_kernel, smem);
   const unsigned grid = (unsigned)((a.m + kCertWarps - 1) / kCertWarps);
   certify_kernel<<<grid, kCertWarps * 32, smem, st>>>(a);
 }
@@ -924,8 +924,7 @@ void launch_certify_batch(const CertifyArgs* tab, const int64_t* row_start, int 
                           int64_t total_rows, cudaStream_t st) {
   if (total_rows <= 0) return;
   const size_t smem = (size_t)kCertWarps * kCertWarpBytes;
-  cudaFuncSetAttribute(certify_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
+  allow_smem(certify_batch_kernel, smem);
   const int rows = cert_batch_rows(total_rows);
   const unsigned grid = (unsigned)((total_rows + rows - 1) / rows);
   certify_batch_kernel<<<grid, kCertWarps * 32, smem, st>>>(tab, row_start, P, total_rows, rows);

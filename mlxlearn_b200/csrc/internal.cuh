@@ -171,6 +171,8 @@ struct QueryPrep {
   float* At;       // [m_pad, dpt] -2*tf32(q - center) (tf32 mode only)
   int* flags;      // [1]: bit 0 = some coordinate outside the screen range
   double* nq;      // [m_pad] ||q - center||^2 (float64), optional
+  int* nonfinite;  // [1]: set when some coordinate is NaN or infinite, optional
+  uint32_t* shared_kth;  // [m_pad] set to "nothing published", optional
 };
 void launch_prep_queries(const Index* ix, const float* Q, int64_t m, int64_t m_pad, int mode,
                          QueryPrep qp, cudaStream_t st);
@@ -188,6 +190,8 @@ struct PrepProblem {
   float* At;                     // [m_pad, dp] (tf32 mode; dp is then the tf32 width)
   double* nq;
   int* flags;
+  int* nonfinite;                // optional
+  uint32_t* shared_kth;          // optional
 };
 PrepProblem prep_problem(const Index* ix, const float* Q, int64_t m, int64_t m_pad, int mode,
                          const QueryPrep& qp);
@@ -228,7 +232,7 @@ int pivot_count(int64_t n);
 int pivot_rows_padded(int P);  // pivots padded to the assignment's tile
 int pivot_dims_padded(int d);  // features padded to its chunk
 void launch_pivots(Index* ix, cudaStream_t st);
-// perm[i] = original row of sorted position i; Qp = Q[perm]
+// perm[i] = original row of sorted position i; Qp = Q[perm]; hist zeroed by the caller
 void launch_query_order(const Index* ix, const float* Q, int64_t m, int* key, int* hist,
                         int* perm, float* Qp, cudaStream_t st);
 // key[r] = nearest pivot of row r of X [n, d] (the index's centre applied);
@@ -424,6 +428,13 @@ bool tensor_map_2d_bf16(CUtensorMap* map, const void* base, uint64_t inner, uint
 bool tensor_map_2d_f32(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer,
                        uint32_t box_inner, uint32_t box_outer, int swizzle_bytes = 128);
 int num_sms(int device);
+// The kernel's dynamic shared memory limit on the current device raised to at
+// least `bytes` (an attribute call only when it was lower: 2 us a launch).
+cudaError_t allow_smem_impl(const void* kernel, size_t bytes);
+template <class Kernel>
+cudaError_t allow_smem(Kernel* kernel, size_t bytes) {
+  return allow_smem_impl(reinterpret_cast<const void*>(kernel), bytes);
+}
 // Polls a screen's bounded waits make before giving up: 2^26 unless
 // B2K_SPIN_LIMIT sets it (tests force the timeout path with it).
 uint32_t device_spin_limit();

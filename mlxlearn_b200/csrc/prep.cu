@@ -305,13 +305,16 @@ __device__ __forceinline__ void prep_query_row_as(const PrepProblem& P, int64_t 
       for (int i = lane; i < dp; i += 32) Ah[row * dp + i] = __float2bfloat16_rn(0.0f);
     if (tf32)
       for (int i = lane; i < dp; i += 32) P.At[row * dp + i] = 0.0f;
-    if (lane == 0) P.E[row] = 0.0f;
+    if (lane == 0) {
+      P.E[row] = 0.0f;
+      if (P.shared_kth) P.shared_kth[row] = 0xffffffffu;
+    }
     return;
   }
   const float* q = P.Q + row * d;
   const int parts = SPLIT ? P.parts : 1;
   double yy = 0.0, hn = 0.0, en = 0.0, pn[3] = {0.0, 0.0, 0.0};
-  bool ok = true;
+  bool ok = true, finite = true;
   if (SPLIT)
     for (int i = operand_cols(d) + lane; i < dp; i += 32)
       Ah[row * dp + i] = __float2bfloat16_rn(0.0f);
@@ -321,6 +324,7 @@ __device__ __forceinline__ void prep_query_row_as(const PrepProblem& P, int64_t 
     const float v = i < d ? q[i] : 0.0f;
     const float c = i < d ? P.center[i] : 0.0f;
     ok &= coord_in_range(v);
+    finite &= (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u;
     const double y = (double)v - (double)c;
     const float h32 = v - c;
     double hv;
@@ -354,6 +358,7 @@ __device__ __forceinline__ void prep_query_row_as(const PrepProblem& P, int64_t 
     for (int t = 0; t < 3; ++t) pn[t] = warp_sum(pn[t]);
   }
   ok = __all_sync(0xffffffffu, ok);
+  finite = ok || __all_sync(0xffffffffu, finite);  // in range implies finite
   if (lane == 0) {
     const double qh = sqrt(hn) * (1.0 + 1e-15);
     const double eq = sqrt(en) * (1.0 + 1e-15) + 0x1p-50 * sqrt(yy);
@@ -382,6 +387,8 @@ __device__ __forceinline__ void prep_query_row_as(const PrepProblem& P, int64_t 
     P.E[row] = __double2float_ru(bound);
     if (P.nq) P.nq[row] = yy;
     if (!ok) atomicOr(P.flags, 1);
+    if (P.shared_kth) P.shared_kth[row] = 0xffffffffu;  // nothing published yet
+    if (P.nonfinite && !finite) atomicOr(P.nonfinite, 1);
   }
 }
 
@@ -515,6 +522,8 @@ PrepProblem prep_problem(const Index* ix, const float* Q, int64_t m, int64_t m_p
   P.At = qp.At;
   P.nq = qp.nq;
   P.flags = qp.flags;
+  P.nonfinite = qp.nonfinite;
+  P.shared_kth = qp.shared_kth;
   return P;
 }
 

@@ -437,7 +437,6 @@ void launch_assign_rows(const Index* ix, const float* X, int64_t n, int* key, in
 void launch_query_order(const Index* ix, const float* Q, int64_t m, int* key, int* hist,
                         int* perm, float* Qp, cudaStream_t st) {
   const int P = ix->n_pivots;
-  cudaMemsetAsync(hist, 0, (size_t)P * sizeof(int), st);
   assign_kernel<<<(unsigned)((m + kAssignThreads - 1) / kAssignThreads), kAssignThreads, 0, st>>>(
       Q, m, ix->d, ix->center, ix->pivots_h, ix->pivot_dpa, ix->pivot_norms, P, key, hist);
   bin_scan_kernel<<<1, 32, 0, st>>>(hist, P);

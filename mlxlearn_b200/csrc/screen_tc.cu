@@ -658,7 +658,7 @@ template <class Sink, bool A_STREAM, int EW, bool BATCH, int KIND = kKindBf16>
 int prepare_tc_variant(int KB_max) {
   const size_t smem = tc_variant_smem<Sink, A_STREAM, EW, BATCH>(KB_max, nullptr);
   auto kern = screen_tc_kernel<Sink, A_STREAM, EW, BATCH, KIND>;
-  return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return (int)allow_smem(kern, smem);
 }
 
 template <class Sink, bool A_STREAM, int EW, bool BATCH, int KIND = kKindBf16>
@@ -671,8 +671,7 @@ int launch_tc_variant(const TcMapSet<BATCH ? kBatchGroups : 1>& maps, const TcPa
   q.a_blocks = KB_max;
   q.spin_limit = device_spin_limit();
   auto kern = screen_tc_kernel<Sink, A_STREAM, EW, BATCH, KIND>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+  const cudaError_t e = allow_smem(kern, smem);
   if (e != cudaSuccess) return (int)e;
   kern<<<grid, tc_block_threads(EW), smem, st>>>(maps, q);
   return (int)cudaGetLastError();

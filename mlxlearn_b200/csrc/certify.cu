@@ -405,7 +405,11 @@ __device__ __forceinline__ int refine_candidates(const CertifyArgs& a, int64_t r
 
 // One query row of one problem, by one warp; `wbase` is the warp's shared
 // memory (kCertWarpBytes).
-__device__ __forceinline__ void certify_row(const CertifyArgs& a, int64_t row, uint8_t* wbase, int lane) {
+// GATHERED: (ci, cv) already hold the `gathered` >= k entries within 2E of the
+// shared k-th value (certify_wide_kernel), of `listed` entries in all.
+template <bool GATHERED = false>
+__device__ __forceinline__ void certify_row(const CertifyArgs& a, int64_t row, uint8_t* wbase,
+                                            int lane, int gathered = 0, unsigned listed = 0) {
   int* ci = reinterpret_cast<int*>(wbase);                          // [kCertifyCap]
   float* cv = reinterpret_cast<float*>(ci + kCertifyCap);           // [kCertifyCap]
   double* cs = reinterpret_cast<double*>(cv + kCertifyCap);         // [kSurvivorCap]
@@ -423,9 +427,9 @@ __device__ __forceinline__ void certify_row(const CertifyArgs& a, int64_t row, u
   // 1. overflow check; the lists' offsets in their concatenation (`hist`,
   // until a radix select needs it)
   bool overflow = false;
-  unsigned entries = 0;
+  unsigned entries = listed;
   const bool flat = S <= kFlatLists;
-  for (int s0 = 0; s0 < S; s0 += 32) {
+  for (int s0 = 0; s0 < S && !GATHERED; s0 += 32) {
     const int s = s0 + lane;
     const int c = s < S ? so.counts[(size_t)s * so.m_pad + row] : 0;
     overflow |= c > so.cap;
@@ -522,9 +526,18 @@ __device__ __forceinline__ void certify_row(const CertifyArgs& a, int64_t row, u
   const int total = S * k;
   float Vk;
   int C = -1;  // candidates, once gathered
-  const uint32_t bound_key = (!so.kth && a.shared_kth) ? a.shared_kth[row] : 0xffffffffu;
-  if (bound_key != 0xffffffffu && (C = gather(__fadd_ru(key_float(bound_key), E2))) >= k &&
-      C <= kCertifyCap) {
+  // So are many lists of the register trackers (more than a warp minimum walks).
+  const uint32_t bound_key = ((!so.kth || S > 32) && a.shared_kth) ? a.shared_kth[row]
+                                                                   : 0xffffffffu;
+  bool cut = GATHERED;
+  if constexpr (GATHERED) {
+    C = gathered;
+  } else if (bound_key != 0xffffffffu) {
+    C = gather(__fadd_ru(key_float(bound_key), E2));
+    cut = C >= k && C <= kCertifyCap;
+    if (!cut) C = -1;
+  }
+  if (cut) {
     __syncwarp();
     auto value_key = [&](int c) { return float_key(cv[c]); };
     Vk = key_float(C <= 32 ? warp_kth_32(lane < C ? value_key(lane) : 0u, C, k, lane)
@@ -548,7 +561,6 @@ __device__ __forceinline__ void certify_row(const CertifyArgs& a, int64_t row, u
     }
     C = w;
   } else if (!so.kth) {
-    C = -1;
     Vk = key_float(warp_radix_select(
         [&](auto f) {
           for (int s = 0; s < S; ++s) {
@@ -730,6 +742,94 @@ __global__ void __launch_bounds__(kCertWarps * 32, 2)
   const int64_t row = (int64_t)blockIdx.x * kCertWarps + w;
   if (row >= a.m) return;
   certify_row(a, row, smem + (size_t)w * kCertWarpBytes, lane);
+}
+
+// Few rows: one block a row gathers the lists (256 threads, a thread a list for
+// the counts, four entries a thread in flight), its first warp does the rest.
+// With a warp a row, one query on 10,000 x 64 (160 lists) spent 62 of its 119 us
+// here; 100,000 x 64, k = 10: 10 queries 0.33 -> 0.16 ms a call, 300 0.33 ->
+// 0.21, 590 0.27 -> 0.21.
+constexpr int kWideThreads = 256;
+constexpr int kWideRows = 800;  // 800: 0.25 -> 0.24 ms, 1,200: 0.24 -> 0.27
+__global__ void __launch_bounds__(kWideThreads)
+    certify_wide_kernel(const __grid_constant__ CertifyArgs a) {
+  extern __shared__ uint8_t smem[];
+  __shared__ unsigned s_sum[kWideThreads / 32];
+  __shared__ int s_count;
+  int* ci = reinterpret_cast<int*>(smem);
+  float* cv = reinterpret_cast<float*>(ci + kCertifyCap);
+  unsigned* off = reinterpret_cast<unsigned*>(smem + kCertWarpBytes) - kFlatLists;  // certify_row's hist
+  const int64_t row = blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const ScreenOut& so = a.scr;
+  const int S = a.S;  // <= kFlatLists (launch_certify)
+  const int c = tid < S ? so.counts[(size_t)tid * so.m_pad + row] : 0;
+  const uint32_t key = a.shared_kth[row];
+  // a screen that gave up left the counts unfinished: certify_row sees the status
+  const int st = a.status ? *reinterpret_cast<volatile const int*>(a.status) : DEV_OK;
+  if (tid == 0) s_count = 0;
+  const bool plain = __syncthreads_or(st != DEV_OK || c > so.cap || c < 0 || key == 0xffffffffu);
+  unsigned entries = 0;
+  if (!plain) {
+    unsigned incl = (unsigned)c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    if (lane == 31) s_sum[w] = incl;
+    __syncthreads();
+    unsigned before = 0;
+    for (int i = 0; i < kWideThreads / 32; ++i) {
+      if (i < w) before += s_sum[i];
+      entries += s_sum[i];
+    }
+    if (tid < S) off[tid] = before + incl - (unsigned)c;
+    __syncthreads();
+    const float limit = __fadd_ru(key_float(key), __fmul_ru(2.0f, a.E[row]));
+    constexpr int kAhead = 4;
+    for (unsigned base = 0; base < entries; base += kWideThreads * kAhead) {
+      int2 e[kAhead];
+      bool in[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const unsigned i = base + kWideThreads * u + tid;
+        in[u] = i < entries;
+        e[u] = make_int2(0, 0);
+        if (in[u]) {
+          int lo = 0, hi = S - 1;  // the last list whose offset is <= i
+          while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (off[mid] <= i)
+              lo = mid;
+            else
+              hi = mid - 1;
+          }
+          e[u] = so.lists[((size_t)lo * so.m_pad + row) * so.cap + (i - off[lo])];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const float v = __int_as_float(e[u].x);
+        const bool pass = in[u] && v <= limit;
+        const unsigned bal = __ballot_sync(0xffffffffu, pass);
+        int pos = 0;
+        if (lane == 0 && bal) pos = atomicAdd(&s_count, __popc(bal));
+        pos = __shfl_sync(0xffffffffu, pos, 0) + __popc(bal & ((1u << lane) - 1));
+        if (pass && pos < kCertifyCap) {
+          ci[pos] = e[u].y;
+          cv[pos] = v;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (w != 0) return;
+  const int C = s_count;
+  if (!plain && C >= a.k && C <= kCertifyCap)
+    certify_row<true>(a, row, smem, lane, C, entries);
+  else
+    certify_row(a, row, smem, lane);
 }
 
 // The block's next row for this warp (its previous row's scratch is free).
@@ -914,6 +1014,12 @@ __global__ void __launch_bounds__(kExactThreads)
 
 void launch_certify(const CertifyArgs& a, cudaStream_t st) {
   if (a.m <= 0) return;
+  // Rows for which a block each is faster: while every block is resident at once
+  // and there are enough lists to share (measured in the comment at the kernel).
+  if (a.m <= kWideRows && a.S > 16 && a.S <= kFlatLists && a.shared_kth) {
+    certify_wide_kernel<<<(unsigned)a.m, kWideThreads, kCertWarpBytes, st>>>(a);
+    return;
+  }
   const size_t smem = (size_t)kCertWarps * kCertWarpBytes;
   allow_smem(certify_kernel, smem);
   const unsigned grid = (unsigned)((a.m + kCertWarps - 1) / kCertWarps);

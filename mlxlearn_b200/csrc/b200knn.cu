@@ -327,7 +327,12 @@ static int make_row_groups(Index& ix) {
   if ((rc = ialloc(ix, &ix.xperm, (size_t)ix.n))) return rc;
   if ((rc = ialloc(ix, &ix.xinv, (size_t)ix.n))) return rc;
   if ((rc = ialloc(ix, &ix.group_start, (size_t)P + 1))) return rc;
-  launch_assign_rows(&ix, ix.X, ix.n, key, hist, st);
+  unsigned long long* best64 = nullptr;
+  if (const size_t words = assign_scratch(&ix, ix.n)) {
+    if ((rc = dalloc(&best64, words, st))) return rc;
+    fr.keep(best64);
+  }
+  launch_assign_rows(&ix, ix.X, ix.n, key, hist, best64, st);
   launch_row_groups(key, ix.n, P, hist, tiles, ix.group_start, ix.xperm, ix.xinv, st);
   B2K_CUDA(cudaGetLastError());
   return B2K_OK;
@@ -705,6 +710,7 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
     Workspace ws;
     int *hist = nullptr, *key = nullptr, *pm = nullptr, *home = nullptr, *seed_counts = nullptr;
     float *Qp = nullptr, *seed_kth = nullptr;
+    unsigned long long* best64 = nullptr;
     uint32_t* shared_kth = nullptr;
     int* fb_list = nullptr;
     QueryPrep qp{};
@@ -717,6 +723,7 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
       ws.reserve(&key, (size_t)m);  // nearest pivot of each query
       ws.reserve(&pm, (size_t)m);
       ws.reserve(&Qp, (size_t)m * ix.d);
+      if (const size_t words = assign_scratch(&ix, m)) ws.reserve(&best64, words);
     }
     ws.reserve(&shared_kth, (size_t)m_pad);
     ws.reserve(&qp.E, (size_t)m_pad);
@@ -744,7 +751,7 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
     const int* perm = ext_perm;
     const float* Qs = dQ;
     if (grouped) {
-      launch_query_order(&ix, dQ, m, key, hist, pm, Qp, st);
+      launch_query_order(&ix, dQ, m, key, hist, best64, pm, Qp, st);
       B2K_CUDA(cudaGetLastError());
       perm = pm;
       Qs = Qp;

@@ -233,12 +233,14 @@ int pivot_rows_padded(int P);  // pivots padded to the assignment's tile
 int pivot_dims_padded(int d);  // features padded to its chunk
 void launch_pivots(Index* ix, cudaStream_t st);
 // perm[i] = original row of sorted position i; Qp = Q[perm]; hist zeroed by the caller
+// best64: assign_scratch(ix, m) words, or null when that is 0
+size_t assign_scratch(const Index* ix, int64_t m);
 void launch_query_order(const Index* ix, const float* Q, int64_t m, int* key, int* hist,
-                        int* perm, float* Qp, cudaStream_t st);
+                        unsigned long long* best64, int* perm, float* Qp, cudaStream_t st);
 // key[r] = nearest pivot of row r of X [n, d] (the index's centre applied);
 // hist[p] = rows per pivot
 void launch_assign_rows(const Index* ix, const float* X, int64_t n, int* key, int* hist,
-                        cudaStream_t st);
+                        unsigned long long* best64, cudaStream_t st);
 // Rows grouped by key, stable: group_start[P + 1], perm (group position -> row)
 // and inv (its inverse).  hist[p] = rows of key p; tiles holds
 // row_group_scratch(n, P) ints.

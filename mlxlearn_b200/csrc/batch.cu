@@ -73,12 +73,11 @@ int64_t rup(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 int kmax_class(int k) { return k <= 8 ? 8 : k <= 12 ? 12 : k <= 16 ? 16 : 64; }
 
 // ---------------------------------------------------------------- tuning
-// Epilogue warps per (dp, heap width) bucket; 0 = the default (16 for the
-// register-heap trackers, 8 for the lazy tracker).
+// Epilogue warps per (dp, heap width) bucket; 0 = the default, 16.
 struct Tuning {
   int ew = 0;
 };
-int default_ew(int kmax) { return kmax <= 16 ? 16 : 8; }
+constexpr int kDefaultEw = 16;
 struct TuneKey {
   int dp, kmax;
   bool operator<(const TuneKey& o) const { return dp != o.dp ? dp < o.dp : kmax < o.kmax; }
@@ -174,8 +173,10 @@ struct b2k_batch {
   // tuned state
   std::vector<b2k::LaunchSpec> specs;
   std::vector<b2k::TcBatchLaunch> launches;
+  std::vector<b2k::TcBatchLaunch> seed_launches;  // before them (seed_tiles_of)
+  b2k::SeedProblem* seed_tab = nullptr;           // [n_graph], or null: no seeding pass
   b2k::CertifyArgs* cert_tab = nullptr;
-  int* item_counters = nullptr;  // [launches]
+  int* item_counters = nullptr;  // [launches + seed_launches]
   int work_items = 0;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -337,6 +338,21 @@ int build_fixed(b2k_batch* b, cudaStream_t st) {
   return B2K_OK;
 }
 
+// Reference tiles a problem's queries scan in the seeding pass: its first few,
+// none for problems of under eight tiles.  Every (split, column group) list of a
+// batch used to fill from nothing; now it starts from the k-th smallest value of
+// this sample, which is no smaller than that of all rows (unrepresentative first
+// tiles only cost speed).  The register trackers refine a list's threshold at
+// every admission, so 1/32 of the rows does (1/16: the same time); the lazy
+// tracker keeps the sample's until a list is full, so its list entries and the
+// certify pass shrink with a larger one.  32 uneven problems: 6.2 ms without the
+// pass and with eight lazy epilogue warps, 5.2 ms with 1/32 for both and sixteen
+// warps, 4.7 with 1/16 for the lazy tracker, 4.5 with 1/8.
+int seed_tiles_of(const BProb& p) {
+  if (p.n_tiles < 8) return 0;
+  return p.kmax == 64 ? std::min(32, (p.n_tiles + 7) / 8) : std::min(8, (p.n_tiles + 31) / 32);
+}
+
 // ------------------------------------------------------------- tuned layout
 Tuning tuning_for(const BProb& p, const std::map<TuneKey, Tuning>& tune) {
   auto it = tune.find(TuneKey{p.dp, p.kmax});
@@ -349,6 +365,8 @@ int build_tuned(b2k_batch* b, const std::map<TuneKey, Tuning>& tune, int gran,
   b->tuned.release();
   b->specs.clear();
   b->launches.clear();
+  b->seed_launches.clear();
+  b->seed_tab = nullptr;
   const int P = b->n_graph;
   if (P == 0) return B2K_OK;
   const int sms = num_sms(b->device);
@@ -358,7 +376,7 @@ int build_tuned(b2k_batch* b, const std::map<TuneKey, Tuning>& tune, int gran,
   for (auto& p : b->probs) {
     if (!p.in_graph) continue;
     const Tuning t = tuning_for(p, tune);
-    p.ew = t.ew ? t.ew : default_ew(p.kmax);
+    p.ew = t.ew ? t.ew : kDefaultEw;
     p.halves = p.ew / 4;
     total_cost += (double)p.m_tiles * p.n_tiles * (p.KB + 1);
     classes[std::make_tuple(p.kmax, p.ew, p.KB > 4)].push_back((int)(&p - b->probs.data()));
@@ -470,6 +488,47 @@ int build_tuned(b2k_batch* b, const std::map<TuneKey, Tuning>& tune, int gran,
   std::vector<const BProb*> by_gi(P);
   for (auto& q : b->probs)
     if (q.in_graph) by_gi[q.gi] = &q;
+  // seeding pass: sixteen values (k for the register trackers) in each of four
+  // column groups a row, no list
+  std::vector<TcProblem> seed_tc(tc);
+  std::vector<SeedProblem> seed(P);
+  size_t seed_rows = 0, seed_vals = 0;
+  for (int gi = 0; gi < P; ++gi) {
+    const BProb& p = *by_gi[gi];
+    SeedProblem& q = seed[gi];
+    q = SeedProblem{nullptr, b->skth + p.pad0, 0, p.m_pad, p.k, p.kmax == 64 ? 16 : p.k};
+    if (!seed_tiles_of(p) || 4 * q.kl < p.k) continue;
+    q.m = (int)p.m;
+    seed_rows += 4 * (size_t)p.m_pad;
+    seed_vals += 4 * (size_t)p.m_pad * q.kl;
+  }
+  TcProblem* d_seed_tc = nullptr;
+  if (seed_rows) {
+    float* d_vals = nullptr;
+    int* d_cnt = nullptr;
+    if ((rc = o.alloc(&d_vals, seed_vals))) return rc;
+    if ((rc = o.alloc(&d_cnt, seed_rows))) return rc;
+    if ((rc = o.alloc(&d_seed_tc, (size_t)P))) return rc;
+    if ((rc = o.alloc(&b->seed_tab, (size_t)P))) return rc;
+    for (int gi = 0; gi < P; ++gi) {
+      SeedProblem& q = seed[gi];
+      if (!q.m) continue;
+      SinkArgs& sink = seed_tc[gi].sink;
+      sink.out.lists = nullptr;
+      sink.out.cap = 0;
+      sink.out.counts = d_cnt;
+      sink.out.kth = d_vals;
+      sink.k = q.kl;
+      sink.shared_kth = nullptr;
+      q.kth = d_vals;
+      d_cnt += 4 * (size_t)q.m_pad;
+      d_vals += 4 * (size_t)q.m_pad * q.kl;
+    }
+    BCUDA(cudaMemcpyAsync(d_seed_tc, seed_tc.data(), P * sizeof(TcProblem),
+                          cudaMemcpyHostToDevice, st));
+    BCUDA(cudaMemcpyAsync(b->seed_tab, seed.data(), P * sizeof(SeedProblem),
+                          cudaMemcpyHostToDevice, st));
+  }
   b->work_items = 0;
   for (auto& spec : b->specs) {
     struct Item {
@@ -521,11 +580,37 @@ int build_tuned(b2k_batch* b, const std::map<TuneKey, Tuning>& tune, int gran,
                          cudaGetErrorString((cudaError_t)pr));
     b->launches.push_back(L);
     b->work_items += (int)flat.size();
+    // the seeding items of the same problems, four epilogue warps a lane group
+    std::vector<int4> seeds;
+    for (int gi : spec.probs)
+      if (seed[gi].m)
+        for (int tt = 0; tt < by_gi[gi]->m_tiles; ++tt)
+          seeds.push_back(make_int4(gi, tt, 0, seed_tiles_of(*by_gi[gi])));
+    if (seeds.empty()) continue;
+    std::stable_sort(seeds.begin(), seeds.end(), [&](const int4& a, const int4& c) {
+      return a.w * (tc[a.x].KB + 1) > c.w * (tc[c.x].KB + 1);
+    });
+    int4* d_seeds = nullptr;
+    if ((rc = o.alloc(&d_seeds, seeds.size()))) return rc;
+    BCUDA(cudaMemcpyAsync(d_seeds, seeds.data(), seeds.size() * sizeof(int4),
+                          cudaMemcpyHostToDevice, st));
+    L.probs = d_seed_tc;
+    L.items = d_seeds;
+    L.n_items = (int)seeds.size();
+    L.grid = (int)std::min<size_t>((size_t)sms, seeds.size());
+    L.kmax = std::min(spec.kmax, 16);
+    L.ew = 16;
+    if (const int ps = prepare_screen_tc_batch(L.kmax, L.ew, L.a_stream, L.KB_max))
+      return bfail(B2K_ECUDA, "batched seeding setup failed: %s",
+                   cudaGetErrorString((cudaError_t)ps));
+    b->seed_launches.push_back(L);
   }
   // one item counter per launch, zeroed at the start of every run
-  if ((rc = o.alloc(&b->item_counters, b->launches.size()))) return rc;
+  if ((rc = o.alloc(&b->item_counters, b->launches.size() + b->seed_launches.size()))) return rc;
   for (size_t i = 0; i < b->launches.size(); ++i)
     b->launches[i].item_counter = b->item_counters + i;
+  for (size_t i = 0; i < b->seed_launches.size(); ++i)
+    b->seed_launches[i].item_counter = b->item_counters + b->launches.size() + i;
   BCUDA(cudaStreamSynchronize(st));
   return B2K_OK;
 }
@@ -536,10 +621,20 @@ int record(b2k_batch* b, cudaStream_t st) {
   if (P == 0) return B2K_OK;
   BCUDA(cudaMemsetAsync(b->zero_block, 0, (8 + (size_t)P) * sizeof(int), st));
   BCUDA(cudaMemsetAsync(b->counters, 0, 4 * sizeof(unsigned long long), st));
-  BCUDA(cudaMemsetAsync(b->item_counters, 0, b->launches.size() * sizeof(int), st));
+  BCUDA(cudaMemsetAsync(b->item_counters, 0,
+                        (b->launches.size() + b->seed_launches.size()) * sizeof(int), st));
   BCUDA(cudaMemsetAsync(b->skth, 0xff, (size_t)b->total_pad * sizeof(uint32_t), st));
   launch_prep_queries_batch(b->prep_tab, b->pad_start, P, b->total_pad, st);
   BCUDA(cudaGetLastError());
+  for (const auto& L : b->seed_launches) {
+    const int lr = launch_screen_tc_batch(L, st);
+    if (lr) return bfail(B2K_ECUDA, "batched seeding launch failed: %s",
+                         cudaGetErrorString((cudaError_t)lr));
+  }
+  if (b->seed_tab) {
+    launch_seed_kth_batch(b->seed_tab, b->row_start, P, b->total_rows, st);
+    BCUDA(cudaGetLastError());
+  }
   for (const auto& L : b->launches) {
     const int lr = launch_screen_tc_batch(L, st);
     if (lr) return bfail(B2K_ECUDA, "batched tcgen05 screen launch failed: %s",
@@ -651,10 +746,10 @@ int autotune(b2k_batch* b, std::map<TuneKey, Tuning>& tune, int& gran) {
   // epilogue width per (dp, heap width) bucket
   for (const TuneKey& k : keys) {
     const Tuning cur = tune.count(k) ? tune[k] : Tuning{};
-    const int ew0 = cur.ew ? cur.ew : default_ew(k.kmax);
+    const int ew0 = cur.ew ? cur.ew : kDefaultEw;
     Tuning keep = cur;
     for (int ew : {16, 8, 4}) {
-      if (ew == ew0 || (ew == 16 && k.kmax > 16)) continue;
+      if (ew == ew0) continue;
       Tuning alt;
       alt.ew = ew;
       tune[k] = alt;

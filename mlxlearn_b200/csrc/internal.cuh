@@ -259,6 +259,16 @@ void launch_home_tiles(const int* perm, const int* key, int64_t m, const int* gr
 void launch_seed_kth(const float* kth, int groups, int kl, int64_t m, int64_t m_pad, int k,
                      uint32_t* shared_kth, cudaStream_t st);
 
+// The batched form: problem p owns global rows [row_start[p], row_start[p + 1]);
+// m = 0 leaves a problem's words alone.
+struct SeedProblem {
+  const float* kth;   // [4][m_pad][kl]
+  uint32_t* shared_kth;
+  int m, m_pad, k, kl;
+};
+void launch_seed_kth_batch(const SeedProblem* tab, const int64_t* row_start, int P,
+                           int64_t total_rows, cudaStream_t st);
+
 // second pass over uncertified rows: Qout[i] = Qs[rows[i]], pout[i] = perm[rows[i]]
 void launch_gather_fallback(const float* Qs, int d, const int* rows, const int* perm, int count,
                             float* Qout, int* pout, cudaStream_t st);

@@ -390,10 +390,9 @@ __global__ void __launch_bounds__(kGroupWarps * 32)
 // One thread per query: the k-th smallest of its G ascending lists of kl values
 // (a k-way merge by list heads) as its shared k-th key; a query with fewer than
 // k finite values keeps its key.
-__global__ void seed_kth_kernel(const float* __restrict__ kth, int G, int kl, int64_t m,
-                                int64_t m_pad, int k, uint32_t* __restrict__ shared_kth) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= m) return;
+__device__ __forceinline__ void seed_kth_row(const float* __restrict__ kth, int G, int kl,
+                                             int64_t r, int64_t m_pad, int k,
+                                             uint32_t* __restrict__ shared_kth) {
   constexpr int kMaxG = 4;
   float head[kMaxG];
   int pos[kMaxG];
@@ -419,6 +418,23 @@ __global__ void seed_kth_kernel(const float* __restrict__ kth, int G, int kl, in
   if (v < INFINITY) shared_kth[r] = float_key(v);
 }
 
+__global__ void seed_kth_kernel(const float* __restrict__ kth, int G, int kl, int64_t m,
+                                int64_t m_pad, int k, uint32_t* __restrict__ shared_kth) {
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < m) seed_kth_row(kth, G, kl, r, m_pad, k, shared_kth);
+}
+
+__global__ void seed_kth_batch_kernel(const SeedProblem* __restrict__ tab,
+                                      const int64_t* __restrict__ row_start, int P,
+                                      int64_t total) {
+  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= total) return;
+  const int p = problem_of(row_start, P, g);
+  const SeedProblem s = tab[p];
+  const int64_t r = g - row_start[p];
+  if (r < s.m) seed_kth_row(s.kth, 4, s.kl, r, s.m_pad, s.k, s.shared_kth);
+}
+
 }  // namespace
 
 size_t row_group_scratch(int64_t n, int P) {
@@ -442,6 +458,13 @@ void launch_seed_kth(const float* kth, int groups, int kl, int64_t m, int64_t m_
   if (m <= 0) return;
   seed_kth_kernel<<<(unsigned)((m + 127) / 128), 128, 0, st>>>(kth, groups, kl, m, m_pad, k,
                                                                shared_kth);
+}
+
+void launch_seed_kth_batch(const SeedProblem* tab, const int64_t* row_start, int P,
+                           int64_t total_rows, cudaStream_t st) {
+  if (total_rows <= 0) return;
+  seed_kth_batch_kernel<<<(unsigned)((total_rows + 127) / 128), 128, 0, st>>>(tab, row_start, P,
+                                                                              total_rows);
 }
 
 void launch_home_tiles(const int* perm, const int* key, int64_t m, const int* group_start,

@@ -819,6 +819,7 @@ int tc_u8_column_groups(int k) { return k <= 8 ? 4 : 2; }
     case 12 * 32 + 4: return CALL(KnnSink<12>, 4);                          \
     case 16 * 32 + 8: return CALL(KnnSink<16>, 8);                          \
     case 16 * 32 + 4: return CALL(KnnSink<16>, 4);                          \
+    case 64 * 32 + 16: return CALL(LazyKnnSink, 16);                        \
     case 64 * 32 + 8: return CALL(LazyKnnSink, 8);                          \
     case 64 * 32 + 4: return CALL(LazyKnnSink, 4);                          \
     default: return (int)cudaErrorInvalidValue;                             \

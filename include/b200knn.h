@@ -291,7 +291,8 @@ typedef struct b2k_radius_result b2k_radius_result;
  * The result is held by the library; read its size with
  * b2k_radius_result_nnz, copy it out with b2k_radius_result_fetch, then
  * release it.  Rows ascend by training index, or by (distance, index) when
- * sort_results is set.
+ * sort_results is 1; 2 leaves them in no particular order, for reductions that
+ * do not depend on it (class counts).
  * Replaces NeighborIndex.query_radius_csr / RadiusSearch.query_with_plan and
  * the Metal screen (src/mlxlearn/_kernels/distance.py:285-342,
  * src/mlxlearn/_kernels/radius.py:380-453,

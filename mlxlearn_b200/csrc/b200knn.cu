@@ -1235,6 +1235,7 @@ static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int ex
   if ((rc = dalloc(&qp.nq, (size_t)m_pad, st))) return rc;
   fr.keep(qp.nq);
   qp.flags = status + 4;
+  qp.nonfinite = status + 5;
   if (tc) {
     if ((rc = dalloc(&qp.Ah, (size_t)m_pad * ix.dp, st))) return rc;
     fr.keep(qp.Ah);
@@ -1269,8 +1270,10 @@ static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int ex
     return fail(B2K_ECUDA, "cuTensorMapEncodeTiled failed for the query rows");
   auto screen = [&](int kind) -> int {
     if (tc) {
+      // status[6], [7] (zeroed above) count the claimed units of the two screens
       int lr = launch_screen_tc(&ix, &tmap_a, m, m_pad, exclude_self, q_offset, S, qp.E, kind,
-                                sa, status, st, qrows);
+                                sa, status, st, qrows,
+                                status + (kind == kSinkRadiusFill ? 7 : 6));
       if (lr) return fail(B2K_ECUDA, "tcgen05 screen launch failed: %s",
                           cudaGetErrorString((cudaError_t)lr));
       return B2K_OK;
@@ -1294,6 +1297,7 @@ static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int ex
   B2K_CUDA(cudaMemcpyAsync(hstatus, status, sizeof(hstatus), cudaMemcpyDeviceToHost, st));
   if (cap) B2K_CUDA(cudaMemcpyAsync(&n_ovf, ovf + m, sizeof(int), cudaMemcpyDeviceToHost, st));
   B2K_CUDA(cudaStreamSynchronize(st));
+  if (hstatus[5]) return fail(B2K_ENONFINITE, "training and query coordinates must be finite");
   if (hstatus[0] != DEV_OK)
     return fail(B2K_ETIMEOUT, "a bounded device wait gave up (code %d)", hstatus[0]);
   if ((hstatus[4] & 1) && !admit_all)
@@ -1487,16 +1491,9 @@ int b2k_radius(b2k_index* h, const float* Q, int64_t m, double radius, int32_t e
     return rc;
   }
   cudaMemcpyAsync(dQ, Q, (size_t)m * ix.d * sizeof(float), cudaMemcpyHostToDevice, st);
-  bool finite = true;
-  rc = device_finite(dQ, (size_t)m * ix.d, st, &finite);
-  if (!rc && !finite) rc = fail(B2K_ENONFINITE, "training and query coordinates must be finite");
-  if (rc) {
-    cudaFreeAsync(dQ, st);
-    delete res;
-    return rc;
-  }
+  // (NaN / inf queries are found by the block's query preparation)
   rc = radius_block(ix, dQ, m, R2, exclude_self, q_offset, need_distance != 0,
-                    sort_results != 0, !ix.range_ok, st, res);
+                    sort_results == 1, !ix.range_ok, st, res, nullptr, false, sort_results != 2);
   cudaFreeAsync(dQ, st);
   cudaStreamSynchronize(st);
   if (rc) {

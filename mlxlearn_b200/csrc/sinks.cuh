@@ -27,6 +27,9 @@ struct SinkArgs {
   int rcap;              // RadiusListSink: entries kept per list
 };
 
+// kWarpWide: every lane of a warp calls every method.  kSmall: few enough
+// registers of state for the epilogue to hold both chunks of a tile.
+
 // Admitted columns of a 32-column chunk as a bit mask (bit i: v[i] <= T),
 // the excluded column (self, when it lies in the chunk) cleared.  The four
 // 8-column group minima come first (3-input minima); only groups
@@ -58,7 +61,7 @@ __device__ __forceinline__ uint32_t admit_mask32(const float (&v)[32], float T, 
 
 template <int KMAX>
 struct KnnSink {
-  static constexpr bool kWarpWide = false;
+  static constexpr bool kWarpWide = false, kSmall = false;
   RowTracker<KMAX> tr;
   size_t slot;
   B2K_DEV void init(const SinkArgs& a, int row, int split, float E, int self) {
@@ -80,7 +83,7 @@ struct KnnSink {
 };
 
 struct RadiusCountSink {
-  static constexpr bool kWarpWide = false;
+  static constexpr bool kWarpWide = false, kSmall = true;
   float T;
   int self, cnt;
   size_t slot;
@@ -101,7 +104,7 @@ struct RadiusCountSink {
 };
 
 struct RadiusFillSink {
-  static constexpr bool kWarpWide = false;
+  static constexpr bool kWarpWide = false, kSmall = true;
   float T;
   int self;
   int* out;
@@ -129,7 +132,7 @@ struct RadiusFillSink {
 // count above it marks a row whose list lost columns (the caller answers that
 // row again with the counted two-pass form).
 struct RadiusListSink {
-  static constexpr bool kWarpWide = false;
+  static constexpr bool kWarpWide = false, kSmall = true;
   float T;
   int self, cnt, cap;
   int* out;
@@ -174,7 +177,7 @@ struct RadiusListSink {
 // inclusive.  The padding rows' v is INT_MAX and never admitted.
 template <int KMAX>
 struct ExactU8Sink {
-  static constexpr bool kWarpWide = false;
+  static constexpr bool kWarpWide = false, kSmall = false;
   int kv[KMAX], kc[KMAX];
   int bound;          // admit v <= bound: min(k-th - 1, shared k-th)
   int shared_v;       // smallest k-th published for this query (INT_MAX: none)
@@ -267,7 +270,7 @@ struct ExactU8Sink {
 // end of the query block; `hist` is the warp's 256-word shared scratch.
 static_assert(kListCap <= 512, "the lazy tracker's warp select holds 16 entries per lane");
 struct LazyKnnSink {
-  static constexpr bool kWarpWide = true;
+  static constexpr bool kWarpWide = true, kSmall = false;
   LazyTracker tr;
   size_t slot;
   unsigned* hist;

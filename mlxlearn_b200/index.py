@@ -276,7 +276,7 @@ class NeighborIndex:
     # ----------------------------------------------------------------- radius
     def query_radius_csr(self, Q, radius, *, need_distance=True, exclude_self=False,
                          sort_results=False, algorithm="auto", n_jobs=None, patched=False,
-                         query_block_size=None, raw=False):
+                         query_block_size=None, raw=False, _any_order=False):
         """Neighbourhoods within an inclusive Euclidean radius, as CSR batches.
 
         A training row is returned iff its exact squared distance is at most
@@ -287,7 +287,8 @@ class NeighborIndex:
         copied if read; otherwise the batches are copied into page-locked
         host memory at once and the device results freed.
         ``algorithm``/``n_jobs``/``patched`` are accepted for signature
-        compatibility.
+        compatibility.  ``_any_order`` leaves the rows unsorted (for class
+        counts, which do not depend on the order).
         """
         from .radius_result import RadiusCSR
 
@@ -311,7 +312,8 @@ class NeighborIndex:
             rc = lib.b2k_radius(h, block.ctypes.data if len(block) else None, stop - start,
                                 float(radius), int(bool(exclude_self)), start,
                                 int(bool(need_distance or sort_results)),
-                                int(bool(sort_results)), ctypes.byref(res))
+                                2 if _any_order and not sort_results else int(bool(sort_results)),
+                                ctypes.byref(res))
             _lib.check(rc, "b2k_radius")
             part = RadiusCSR.from_device(res, stop - start, device=self.device,
                                          distances=bool(need_distance))
@@ -323,18 +325,22 @@ class NeighborIndex:
         return parts
 
     def query_radius_reduce(self, Q, radius, *, codes=None, n_classes=0, targets=None,
-                            weighted=False, exclude_self=False, query_block_size=None):
+                            weighted=False, exclude_self=False, query_block_size=None,
+                            _proba=False):
         """Per-query class votes (``codes``: CUDA int32 labels of the training
         rows) or target means (``targets``: CUDA float64) over the radius
         neighbourhoods, reduced on the device without downloading them.
         Returns ``(votes [m, n_classes] or means [m], counts [m])`` as numpy
-        arrays, equal to the host reductions over :meth:`query_radius_csr`."""
+        arrays, equal to the host reductions over :meth:`query_radius_csr`.
+        ``_proba`` (unweighted codes) divides each row's votes by its count on
+        the device (rows without neighbours stay zero)."""
         if (codes is None) == (targets is None):
             raise ValueError("pass exactly one of codes and targets")
         parts = self.query_radius_csr(Q, radius, need_distance=bool(weighted),
                                       exclude_self=exclude_self,
-                                      query_block_size=query_block_size, raw=True)
-        pieces = [p.votes(codes, n_classes, weighted) if codes is not None
+                                      query_block_size=query_block_size, raw=True,
+                                      _any_order=codes is not None and not weighted)
+        pieces = [p.votes(codes, n_classes, weighted, _proba) if codes is not None
                   else p.mean(targets, weighted) for p in parts]
         for p in parts:
             p.release()
@@ -349,7 +355,8 @@ class NeighborIndex:
         counts, as numpy int64 arrays: the argmax of the normalised votes,
         computed on the device without downloading the votes."""
         parts = self.query_radius_csr(Q, radius, need_distance=False, exclude_self=exclude_self,
-                                      query_block_size=query_block_size, raw=True)
+                                      query_block_size=query_block_size, raw=True,
+                                      _any_order=True)
         pieces = [p.predict_codes(codes, n_classes) for p in parts]
         for p in parts:
             p.release()

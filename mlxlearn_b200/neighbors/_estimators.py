@@ -242,11 +242,13 @@ class RadiusNeighborsClassifier(RadiusMixin, NeighborsMixin, ClassifierMixin, Ba
         # votes reduced on the device from the device neighbourhoods
         votes, counts = self._index_.query_radius_reduce(
             Q, self.radius, codes=self._codes_device(), n_classes=len(self.classes_),
-            weighted=weighted, exclude_self=query_is_train)
+            weighted=weighted, exclude_self=query_is_train, _proba=not weighted)
         self._last_query_backend = "cuda"
         outliers, match = self._outliers(counts, stacklevel=4)  # user -> predict* -> _proba
         if match is not None:
             votes[outliers, match] = 1.0
+        if not weighted:
+            return votes  # divided by the row's count already; an outlier's row sums to 0 or 1
         normalizer = votes.sum(axis=1)[:, None]
         normalizer[normalizer == 0.0] = 1.0
         votes /= normalizer

@@ -139,7 +139,7 @@ class RadiusCSR:
         return np.arange(self._m, dtype=np.int64).repeat(self.lengths())
 
     # ---------------------------------------------------- device reductions
-    def _reduce(self, values, kind: str, n_classes: int, weighted: bool):
+    def _reduce(self, values, kind: str, n_classes: int, weighted: bool, proba: bool = False):
         import torch
 
         if self._handle is None:
@@ -171,13 +171,21 @@ class RadiusCSR:
                                                  int(bool(weighted)), out.data_ptr(),
                                                  counts.data_ptr(), stream)
             _lib.check(rc, "radius reduction")
-        return out.cpu().numpy(), counts.cpu().numpy()
+        if proba:
+            # integer votes: their sum is the count, and the division rounds as
+            # numpy's does
+            out /= counts.clamp(min=1).unsqueeze(1)
+        host = _page_locked(out.numel(), np.float64)
+        torch.from_numpy(host).copy_(out.view(-1))
+        return host.reshape(out.shape), counts.cpu().numpy()
 
-    def votes(self, codes, n_classes: int, weighted: bool):
+    def votes(self, codes, n_classes: int, weighted: bool, proba: bool = False):
         """Per-row class votes (float64 ``[m, n_classes]``: weight 1, or 1/d
         with a row's zero distances taking their 0/1 indicator) and neighbour
-        counts, summed on the device in ascending training-index order."""
-        return self._reduce(codes, "votes", int(n_classes), weighted)
+        counts, summed on the device in ascending training-index order (the
+        counts of weight 1 do not depend on the order).  ``proba`` (weight 1)
+        divides each row by its neighbour count on the device."""
+        return self._reduce(codes, "votes", int(n_classes), weighted, proba and not weighted)
 
     def predict_codes(self, codes, n_classes: int):
         """Per-row first maximum of the class counts (ties -> smallest code,

@@ -112,6 +112,12 @@ B2K_API int b2k_index_download(const b2k_index *index, float *X);
 /* Device pointer of the owned float32 rows [n, d] (valid until destroy). */
 B2K_API const float *b2k_index_device_data(const b2k_index *index);
 
+/* Copy `bytes` of host memory to device memory on `stream` (of the current
+ * device).  Pageable memory is staged through page-locked slots by a few host
+ * threads while an index lives; the source may be reused on return.  No
+ * counterpart in the reference (MLX arrays share memory with the host). */
+B2K_API int b2k_upload(void *d_dst, const void *src, int64_t bytes, void *stream);
+
 /* -------------------------------------------------------------------- kNN */
 
 /* k nearest training rows of each of m host queries Q[m, d].

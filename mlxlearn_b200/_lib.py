@@ -100,6 +100,7 @@ SIGNATURES = {
     "b2k_index_shape": (ctypes.c_int, [_vp, ctypes.POINTER(_i64), ctypes.POINTER(_i32)]),
     "b2k_index_download": (ctypes.c_int, [_vp, _vp]),
     "b2k_index_device_data": (_vp, [_vp]),
+    "b2k_upload": (ctypes.c_int, [_vp, _vp, _i64, _vp]),
     "b2k_knn": (ctypes.c_int, [_vp, _vp, _i64, _i32, _i32, _i64, _i32, _vp, _vp,
                                ctypes.POINTER(Stats)]),
     "b2k_knn_device": (ctypes.c_int, [_vp, _vp, _i64, _i32, _i32, _i64, _i32, _vp, _vp, _vp,

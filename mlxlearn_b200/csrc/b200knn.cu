@@ -1010,6 +1010,8 @@ static int build_from_device(b2k_index* h, const float* src, cudaMemcpyKind kind
   Index& ix = h->ix;
   B2K_CUDA(cudaSetDevice(ix.device));
   keep_pool(ix.device);
+  staging_acquire(ix.device);
+  ix.staging = true;
   B2K_CUDA(cudaStreamCreateWithFlags(&ix.stream, cudaStreamNonBlocking));
   const size_t bytes = (size_t)ix.n * ix.d * sizeof(float);
   int rc;
@@ -1029,7 +1031,10 @@ static int build_from_device(b2k_index* h, const float* src, cudaMemcpyKind kind
     cudaEventDestroy(ready);
     B2K_CUDA(e);
   }
-  B2K_CUDA(cudaMemcpyAsync(ix.X, src, bytes, kind, ix.stream));
+  if (kind == cudaMemcpyHostToDevice)
+    B2K_CUDA(upload_host(ix.X, src, bytes, ix.stream));
+  else
+    B2K_CUDA(cudaMemcpyAsync(ix.X, src, bytes, kind, ix.stream));
   return finish_index(ix, ix.stream);
 }
 
@@ -1094,6 +1099,7 @@ int b2k_index_destroy(b2k_index* h) {
   cudaFree(ix.Xu);
   cudaFree(ix.nxu);
   if (ix.stream) cudaStreamDestroy(ix.stream);
+  if (ix.staging) staging_release(ix.device);
   delete h;
   return B2K_OK;
 }
@@ -1156,7 +1162,7 @@ int b2k_knn(b2k_index* h, const float* Q, int64_t m, int32_t k, int32_t exclude_
     if ((rc = dalloc(&dd, (size_t)m * k, st))) return rc;
     fr.keep(dd);
   }
-  B2K_CUDA(cudaMemcpyAsync(dQ, Q, (size_t)m * ix.d * sizeof(float), cudaMemcpyHostToDevice, st));
+  B2K_CUDA(upload_host(dQ, Q, (size_t)m * ix.d * sizeof(float), st));
   // finiteness is checked on the device inside the search (one pass over HBM)
   rc = knn_device_impl(ix, dQ, m, k, exclude_self, q_offset, mode, dd, di, st, stats);
   if (rc) return rc;
@@ -1490,7 +1496,11 @@ int b2k_radius(b2k_index* h, const float* Q, int64_t m, double radius, int32_t e
     delete res;
     return rc;
   }
-  cudaMemcpyAsync(dQ, Q, (size_t)m * ix.d * sizeof(float), cudaMemcpyHostToDevice, st);
+  if (const cudaError_t e = upload_host(dQ, Q, (size_t)m * ix.d * sizeof(float), st)) {
+    cudaFreeAsync(dQ, st);
+    delete res;
+    return fail(B2K_ECUDA, "upload of the queries: %s", cudaGetErrorString(e));
+  }
   // (NaN / inf queries are found by the block's query preparation)
   rc = radius_block(ix, dQ, m, R2, exclude_self, q_offset, need_distance != 0,
                     sort_results == 1, !ix.range_ok, st, res, nullptr, false, sort_results != 2);

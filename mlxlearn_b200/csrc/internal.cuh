@@ -128,6 +128,7 @@ struct Index {
   // every buffer above but the u8 ones, and whether it came from the
   // stream-ordered pool
   std::vector<std::pair<void*, bool>> owned;
+  bool staging = false;  // counted as a user of the upload staging (upload.cu)
   std::mutex mu;
 };
 
@@ -406,6 +407,13 @@ int knn_backward(const float* Q, int64_t m, const float* X, int64_t n, int d, in
                  const int64_t* idx, const float* G, const float* E, int squared, float* dQ,
                  float* dX, int* workspace, cudaStream_t st);
 size_t knn_backward_workspace_ints(int64_t m, int64_t n, int k);
+
+// ---------------------------------------------------------- uploads (upload.cu)
+// Host to device copy on `st` of the current device; pageable sources go through
+// pinned staging while some index holds it.  The source may be reused on return.
+cudaError_t upload_host(void* dst, const void* src, size_t bytes, cudaStream_t st);
+void staging_acquire(int device);
+void staging_release(int device);
 
 // helpers
 int report_error(int code, const char* msg);  // sets b2k_last_error(), returns code

@@ -79,7 +79,12 @@ class KNeighborsClassifier(NeighborsMixin, ClassifierMixin, BaseEstimator):
         if codes is None:
             codes = torch.from_numpy(self._y.astype(np.int32)).to(dev)
             self.__dict__["_codes_dev"] = codes
-        Qd = torch.from_numpy(np.ascontiguousarray(Q)).to(dev)
+        Q = np.ascontiguousarray(Q)
+        Qd = torch.empty(Q.shape, dtype=torch.float32, device=dev)
+        with torch.cuda.device(dev):
+            _lib.check(_lib.load().b2k_upload(Qd.data_ptr(), Q.ctypes.data, Q.nbytes,
+                                              torch.cuda.current_stream(dev).cuda_stream),
+                       "b2k_upload")
         dist, idx = self._index_.query_device(Qd, k, return_distance=weighted,
                                               exclude_self=query_is_train)
         m, n_classes = idx.shape[0], len(self.classes_)

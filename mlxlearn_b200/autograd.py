@@ -127,6 +127,8 @@ class KnnSegmentDistances(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, Q, X, q_sizes, x_sizes, k, exclude_self, squared):
+        import numpy as np
+
         if not (Q.is_cuda and X.is_cuda):
             raise TypeError("knn_segments expects CUDA tensors")
         Qc = Q.detach().to(torch.float32).contiguous()
@@ -135,10 +137,11 @@ class KnnSegmentDistances(torch.autograd.Function):
         dist64, idx = _segments_forward(Qc, Xc, q_sizes, x_sizes, k, exclude_self)
         xo = _offsets(x_sizes)
         # global reference rows for the backward
-        starts = torch.as_tensor(xo[:-1], device=Qc.device)
-        seg = torch.repeat_interleave(torch.arange(len(q_sizes), device=Qc.device),
-                                      torch.as_tensor(q_sizes, device=Qc.device))
-        gidx = idx + starts[seg].unsqueeze(1)
+        starts, sizes = torch.as_tensor(np.stack([xo[:-1], np.asarray(q_sizes, np.int64)]),
+                                        device=Qc.device)
+        # (with its output size known, no read back of the sizes)
+        gidx = idx + torch.repeat_interleave(starts, sizes,
+                                             output_size=Qc.shape[0]).unsqueeze(1)
         e = dist64.to(torch.float32)
         out = dist64.square().to(torch.float32) if squared else e
         ctx.save_for_backward(Qc, Xc, gidx, e)

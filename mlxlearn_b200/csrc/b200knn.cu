@@ -1189,16 +1189,18 @@ struct b2k_radius_result {
 namespace b2k {
 
 // Entries per list of the single-pass radius screen: B2K_RADIUS_CAP when set
-// (0 = the counted two-pass form), else what a 512 MB budget for the block's
+// (0 = the counted two-pass form), else what a 2 GB budget for the block's
 // lists allows (B2K_RADIUS_LIST_MB), a multiple of 32 in [64, 1024], or 0 when
-// that budget holds fewer than 64 per list.
+// that budget holds fewer than 64 per list.  With 512 MB a few dense rows of
+// 100,003 x 24 (30,011 queries) and 200,000 x 32 (50,000) overflowed, and their
+// counted sub-call cost 0.25 of 2.57 ms and 0.2 of 4.55.
 static int radius_list_cap(int S_lists, int64_t m_pad) {
   if (const char* e = getenv("B2K_RADIUS_CAP")) {
     const long c = atol(e);
     return c <= 0 ? 0 : (int)std::min<long>(c, 1 << 20);
   }
   const char* mb = getenv("B2K_RADIUS_LIST_MB");
-  const int64_t budget = (int64_t)(mb ? atoll(mb) : 512) << 20;
+  const int64_t budget = (int64_t)(mb ? atoll(mb) : 2048) << 20;
   int64_t c = budget / ((int64_t)S_lists * m_pad * (int64_t)sizeof(int)) / 32 * 32;
   return c < 64 ? 0 : (int)std::min<int64_t>(c, 1024);
 }
@@ -1227,50 +1229,42 @@ static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int ex
   const int S_lists = S * (tc ? tc_radius_groups() : simt_column_groups(kSinkRadiusCount));
   const int cap = (tc && !counted) ? radius_list_cap(S_lists, m_pad) : 0;
 
-  int* status = nullptr;
-  if ((rc = dalloc(&status, 8, st))) return rc;
-  fr.keep(status);
-  unsigned long long* counters = nullptr;
-  if ((rc = dalloc(&counters, 2, st))) return rc;
-  fr.keep(counters);
-  B2K_CUDA(cudaMemsetAsync(status, 0, 8 * sizeof(int), st));
-  B2K_CUDA(cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), st));
+  // the block's state, zeroed and read back as one; counters: [0] exact tests,
+  // [2] overflowed rows, [3] candidates, [4] members
+  CallState* state = nullptr;
   QueryPrep qp{};
-  if ((rc = dalloc(&qp.E, (size_t)m_pad, st))) return rc;
-  fr.keep(qp.E);
-  if ((rc = dalloc(&qp.nq, (size_t)m_pad, st))) return rc;
-  fr.keep(qp.nq);
+  float* thr = nullptr;
+  SinkArgs sa{};
+  int64_t *roff = nullptr, *scan_scratch = nullptr;
+  int* ovf = nullptr;  // single pass: overflowed rows [m] + their count
+  Workspace ws;
+  ws.reserve(&state, 1);
+  ws.reserve(&qp.E, (size_t)m_pad);
+  ws.reserve(&qp.nq, (size_t)m_pad);
+  if (tc) ws.reserve(&qp.Ah, (size_t)m_pad * ix.dp);
+  ws.reserve(&thr, (size_t)m_pad);
+  ws.reserve(&sa.rcount, (size_t)S_lists * m_pad);
+  ws.reserve(&roff, (size_t)S_lists * m_pad + 1);
+  if (cap) {
+    ws.reserve(&sa.rcols, (size_t)S_lists * m_pad * cap);
+    ws.reserve(&ovf, (size_t)m + 1);
+  }
+  ws.reserve(&scan_scratch, (size_t)scan_scratch_len(m));  // count offsets, then indptr
+  if ((rc = ws.place(st, fr))) return rc;
+  int* status = state->status;
+  unsigned long long* counters = state->counters;
+  B2K_CUDA(cudaMemsetAsync(state, 0, sizeof(CallState), st));
   qp.flags = status + 4;
   qp.nonfinite = status + 5;
-  if (tc) {
-    if ((rc = dalloc(&qp.Ah, (size_t)m_pad * ix.dp, st))) return rc;
-    fr.keep(qp.Ah);
-  }
   launch_prep_queries(&ix, dQ, m, m_pad, mode, qp, st);
-  float* thr = nullptr;
-  if ((rc = dalloc(&thr, (size_t)m_pad, st))) return rc;
-  fr.keep(thr);
   launch_radius_threshold(qp.nq, qp.E, m, m_pad, admit_all ? INFINITY : R2, thr, st);
   B2K_CUDA(cudaGetLastError());
 
-  SinkArgs sa{};
   sa.thr = thr;
   sa.m_pad = (int)m_pad;
   sa.rcap = cap;
-  if ((rc = dalloc(&sa.rcount, (size_t)S_lists * m_pad, st))) return rc;
-  fr.keep(sa.rcount);
-  int64_t* roff = nullptr;
-  if ((rc = dalloc(&roff, (size_t)S_lists * m_pad + 1, st))) return rc;
-  fr.keep(roff);
   sa.roff = roff;
-  int* ovf = nullptr;  // single pass: overflowed rows [m] + their count
-  if (cap) {
-    if ((rc = dalloc(&sa.rcols, (size_t)S_lists * m_pad * cap, st))) return rc;
-    fr.keep(sa.rcols);
-    if ((rc = dalloc(&ovf, (size_t)m + 1, st))) return rc;
-    fr.keep(ovf);
-    B2K_CUDA(cudaMemsetAsync(ovf + m, 0, sizeof(int), st));
-  }
+  if (cap) B2K_CUDA(cudaMemsetAsync(ovf + m, 0, sizeof(int), st));
   CUtensorMap tmap_a;
   if (tc && !tensor_map_2d_bf16(&tmap_a, qp.Ah, (uint64_t)ix.dp, (uint64_t)m_pad, kTcBK, kTcBM))
     return fail(B2K_ECUDA, "cuTensorMapEncodeTiled failed for the query rows");
@@ -1290,19 +1284,18 @@ static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int ex
   };
   if ((rc = screen(cap ? kSinkRadiusList : kSinkRadiusCount))) return rc;
   if (cap) launch_radius_overflow(sa.rcount, S_lists, m, m_pad, cap, ovf, st);
-  int64_t* scan_scratch = nullptr;  // multi-block scans (count offsets, then indptr)
-  if ((rc = dalloc(&scan_scratch, (size_t)scan_scratch_len(m), st))) return rc;
-  fr.keep(scan_scratch);
   launch_scan_split_counts(sa.rcount, S_lists, m, m_pad, roff, roff + (size_t)S_lists * m_pad,
                            scan_scratch, st);
-  int64_t ncand = 0;
-  int hstatus[8];
-  int n_ovf = 0;
-  B2K_CUDA(cudaMemcpyAsync(&ncand, roff + (size_t)S_lists * m_pad, sizeof(int64_t),
-                           cudaMemcpyDeviceToHost, st));
-  B2K_CUDA(cudaMemcpyAsync(hstatus, status, sizeof(hstatus), cudaMemcpyDeviceToHost, st));
-  if (cap) B2K_CUDA(cudaMemcpyAsync(&n_ovf, ovf + m, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CallState h;
+  const int* hstatus = h.status;
+  B2K_CUDA(cudaMemcpyAsync(counters + 3, roff + (size_t)S_lists * m_pad, sizeof(int64_t),
+                           cudaMemcpyDeviceToDevice, st));
+  if (cap)
+    B2K_CUDA(cudaMemcpyAsync(counters + 2, ovf + m, sizeof(int), cudaMemcpyDeviceToDevice, st));
+  B2K_CUDA(cudaMemcpyAsync(&h, state, sizeof(h), cudaMemcpyDeviceToHost, st));
   B2K_CUDA(cudaStreamSynchronize(st));
+  const int64_t ncand = (int64_t)h.counters[3];
+  const int n_ovf = (int)h.counters[2];
   if (hstatus[5]) return fail(B2K_ENONFINITE, "training and query coordinates must be finite");
   if (hstatus[0] != DEV_OK)
     return fail(B2K_ETIMEOUT, "a bounded device wait gave up (code %d)", hstatus[0]);
@@ -1382,12 +1375,11 @@ static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int ex
   if ((rc = dalloc(&indptr, (size_t)m + 1, st))) return rc;
   launch_scan_rows(ra.mcount, m, indptr, scan_scratch, st);
   B2K_CUDA(cudaGetLastError());
-  int64_t nnz = 0;
-  unsigned long long hc[2];
-  B2K_CUDA(cudaMemcpyAsync(&nnz, indptr + m, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  B2K_CUDA(cudaMemcpyAsync(hc, counters, sizeof(hc), cudaMemcpyDeviceToHost, st));
-  B2K_CUDA(cudaMemcpyAsync(hstatus, status, sizeof(hstatus), cudaMemcpyDeviceToHost, st));
+  B2K_CUDA(cudaMemcpyAsync(counters + 4, indptr + m, sizeof(int64_t), cudaMemcpyDeviceToDevice,
+                           st));
+  B2K_CUDA(cudaMemcpyAsync(&h, state, sizeof(h), cudaMemcpyDeviceToHost, st));
   B2K_CUDA(cudaStreamSynchronize(st));
+  const int64_t nnz = (int64_t)h.counters[4];
   if (hstatus[0] != DEV_OK) {  // the fill pass gave up (classify skipped its rows)
     cudaFreeAsync(indptr, st);
     return fail(B2K_ETIMEOUT, "a bounded device wait gave up (code %d)", hstatus[0]);
@@ -1450,7 +1442,7 @@ static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int ex
   res->indptr = indptr;
   res->indices = indices;
   res->dist = dist;
-  res->exact_tests = (int64_t)hc[0] + (sub ? sub->exact_tests : 0);
+  res->exact_tests = (int64_t)h.counters[0] + (sub ? sub->exact_tests : 0);
   res->candidates = ncand + (sub ? sub->candidates : 0);
   return B2K_OK;
 }

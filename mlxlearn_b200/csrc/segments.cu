@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cstdio>
+#include <cstring>
 #include <vector>
 
 #include "common.cuh"
@@ -593,10 +594,16 @@ extern "C" B2K_API int b2k_knn_segments(const float* dQ, const float* dX, int32_
   int rc = B2K_OK;
   int hflags[16];
   do {
-    if ((e = cudaMemcpyAsync(qseg, q_offsets, off_b, cudaMemcpyHostToDevice, st)) ||
-        (e = cudaMemcpyAsync(xseg, x_offsets, off_b, cudaMemcpyHostToDevice, st)) ||
-        (e = cudaMemcpyAsync(dblocks, blocks.data(), blk_b, cudaMemcpyHostToDevice, st)) ||
-        (e = cudaMemcpyAsync(tab, ex.data(), tab_b, cudaMemcpyHostToDevice, st)) ||
+    // offsets, block list and table lie together: one copy
+    std::vector<unsigned char> up((size_t)(reinterpret_cast<unsigned char*>(fb) - base));
+    auto put = [&](void* at, const void* from, size_t n) {
+      memcpy(up.data() + (static_cast<unsigned char*>(at) - base), from, n);
+    };
+    put(qseg, q_offsets, off_b);
+    put(xseg, x_offsets, off_b);
+    put(dblocks, blocks.data(), blk_b);
+    put(tab, ex.data(), tab_b);
+    if ((e = cudaMemcpyAsync(base, up.data(), up.size(), cudaMemcpyHostToDevice, st)) ||
         (e = cudaMemsetAsync(flags, 0, 16 * sizeof(int), st)) ||
         (e = cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), st))) {
       rc = seg_fail(B2K_ECUDA, "b2k_knn_segments: copy to the device failed");

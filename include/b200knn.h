@@ -293,12 +293,14 @@ B2K_API int b2k_batch_submit(const b2k_problem *problems, int32_t count, void *s
 
 typedef struct b2k_radius_result b2k_radius_result;
 
+#define B2K_RADIUS_ANY_ORDER 0x40000000
+
 /* Every training row within `radius` (inclusive, exact) of each host query.
  * The result is held by the library; read its size with
  * b2k_radius_result_nnz, copy it out with b2k_radius_result_fetch, then
  * release it.  Rows ascend by training index, or by (distance, index) when
- * sort_results is 1; 2 leaves them in no particular order, for reductions that
- * do not depend on it (class counts).
+ * sort_results is set; B2K_RADIUS_ANY_ORDER leaves them in no particular order,
+ * for reductions that do not depend on it (class counts).
  * Replaces NeighborIndex.query_radius_csr / RadiusSearch.query_with_plan and
  * the Metal screen (src/mlxlearn/_kernels/distance.py:285-342,
  * src/mlxlearn/_kernels/radius.py:380-453,

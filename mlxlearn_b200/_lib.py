@@ -88,6 +88,7 @@ class BatchStats(ctypes.Structure):
 
 
 BATCH_AUTOTUNE = 1
+RADIUS_ANY_ORDER = 0x40000000
 
 # Every exported symbol of the C ABI, with (restype, argtypes).
 _vp, _i32, _i64, _dbl = ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_double

@@ -1495,7 +1495,8 @@ int b2k_radius(b2k_index* h, const float* Q, int64_t m, double radius, int32_t e
   }
   // (NaN / inf queries are found by the block's query preparation)
   rc = radius_block(ix, dQ, m, R2, exclude_self, q_offset, need_distance != 0,
-                    sort_results == 1, !ix.range_ok, st, res, nullptr, false, sort_results != 2);
+                    sort_results != 0 && sort_results != B2K_RADIUS_ANY_ORDER, !ix.range_ok, st,
+                    res, nullptr, false, sort_results != B2K_RADIUS_ANY_ORDER);
   cudaFreeAsync(dQ, st);
   cudaStreamSynchronize(st);
   if (rc) {

@@ -312,7 +312,8 @@ class NeighborIndex:
             rc = lib.b2k_radius(h, block.ctypes.data if len(block) else None, stop - start,
                                 float(radius), int(bool(exclude_self)), start,
                                 int(bool(need_distance or sort_results)),
-                                2 if _any_order and not sort_results else int(bool(sort_results)),
+                                _lib.RADIUS_ANY_ORDER if _any_order and not sort_results
+                                else int(bool(sort_results)),
                                 ctypes.byref(res))
             _lib.check(rc, "b2k_radius")
             part = RadiusCSR.from_device(res, stop - start, device=self.device,

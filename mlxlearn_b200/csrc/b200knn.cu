@@ -324,17 +324,22 @@ static int make_row_groups(Index& ix) {
   fr.keep(hist);
   if ((rc = dalloc(&tiles, row_group_scratch(ix.n, P), st))) return rc;
   fr.keep(tiles);
-  if ((rc = ialloc(ix, &ix.xperm, (size_t)ix.n))) return rc;
-  if ((rc = ialloc(ix, &ix.xinv, (size_t)ix.n))) return rc;
-  if ((rc = ialloc(ix, &ix.group_start, (size_t)P + 1))) return rc;
+  int *perm = nullptr, *inv = nullptr, *start = nullptr;
+  if ((rc = ialloc(ix, &perm, (size_t)ix.n))) return rc;
+  if ((rc = ialloc(ix, &inv, (size_t)ix.n))) return rc;
+  if ((rc = ialloc(ix, &start, (size_t)P + 1))) return rc;
   unsigned long long* best64 = nullptr;
   if (const size_t words = assign_scratch(&ix, ix.n)) {
     if ((rc = dalloc(&best64, words, st))) return rc;
     fr.keep(best64);
   }
   launch_assign_rows(&ix, ix.X, ix.n, key, hist, best64, st);
-  launch_row_groups(key, ix.n, P, hist, tiles, ix.group_start, ix.xperm, ix.xinv, st);
+  launch_row_groups(key, ix.n, P, hist, tiles, start, perm, inv, st);
   B2K_CUDA(cudaGetLastError());
+  // (set together: a failed build leaves the index ungrouped)
+  ix.xperm = perm;
+  ix.xinv = inv;
+  ix.group_start = start;
   return B2K_OK;
 }
 

@@ -738,6 +738,11 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
     // the register trackers' lists hold 4 x kListCap entries per (split, query)
     // whatever the column groups (the lazy tracker's select is sized for kListCap)
     so.cap = (tc && !lazy) ? kListCap * 4 / tc_column_groups(k) : kListCap;
+    // (half of it in four lists a split where that would pass 32 GB, from about
+    // two million queries: two lists of kListCap were as large)
+    if (lazy && tc_column_groups(k) == 4 &&
+        (size_t)S_lists * m_pad * kListCap * sizeof(int2) > ((size_t)32 << 30))
+      so.cap = kListCap / 2;
     so.m_pad = (int)m_pad;
     ws.reserve(&so.lists, (size_t)S_lists * m_pad * so.cap);
     ws.reserve(&so.counts, (size_t)S_lists * m_pad);

@@ -392,8 +392,10 @@ int build_tuned(b2k_batch* b, const std::map<TuneKey, Tuning>& tune, int gran,
     p.tps = (p.n_tiles + S - 1) / S;
     p.S = (p.n_tiles + p.tps - 1) / p.tps;
     p.S_lists = p.S * p.halves;
-    // a list never holds more than the columns its slot scans
-    p.cap = (int)std::min<int64_t>(kListCap, (int64_t)p.tps * kTcBN / p.halves);
+    // a list never holds more than the columns its slot scans; the lazy
+    // tracker's hold kListCap for two column groups a split
+    const int full = p.kmax == 64 ? std::min(kListCap, 2 * kListCap / p.halves) : kListCap;
+    p.cap = (int)std::min<int64_t>(full, (int64_t)p.tps * kTcBN / p.halves);
     p.lists_off = lists;
     p.counts_off = counts;
     p.kth_off = kth;

@@ -711,6 +711,21 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
     const bool seed = tc && grouped && ix.group_start && n_tiles >= 2 * kSeedTiles &&
                       seed_enabled();
     const int seed_k = lazy ? 16 : k, seed_groups = tc ? tc_column_groups(seed_k) : 0;
+    // Lazy lists without grouped queries (m < 2048 or few rows) are seeded from
+    // windows spread over the rows: an eighth of the tiles, 4 to 64 (128 where the
+    // units would otherwise leave SMs idle), in as many windows as keep two units
+    // an SM, at least 8.  Unseeded, a split's list sees fewer columns than it holds
+    // and keeps them all, and the certify pass walks every row of the index
+    // (100,000 x 20, 100 queries, k = 50: 100,000 entries a row and 1.87 ms, seeded
+    // 465 and 0.15; 500,000 x 3, k = 17: 1.31 -> 0.56; 5,000 x 8, 5,000 queries,
+    // k = 50: 0.86 -> 0.23).
+    const bool spread = lazy && !seed && n_tiles >= 8 && seed_enabled();
+    const int spread_most = (int)std::min<int64_t>(128, std::max<int64_t>(64, sms / (m_pad / bm)));
+    const int spread_tiles =
+        (int)std::min<int64_t>(spread_most, std::max<int64_t>(4, n_tiles / 8));
+    const int spread_S = (int)std::min<int64_t>(
+        spread_tiles, std::max<int64_t>(8, 2 * sms / (m_pad / bm)));
+    const int spread_window = (spread_tiles + spread_S - 1) / spread_S;
 
     Workspace ws;
     int *hist = nullptr, *key = nullptr, *pm = nullptr, *home = nullptr, *seed_counts = nullptr;
@@ -739,18 +754,20 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
     // whatever the column groups (the lazy tracker's select is sized for kListCap)
     so.cap = (tc && !lazy) ? kListCap * 4 / tc_column_groups(k) : kListCap;
     // (half of it in four lists a split where that would pass 32 GB, from about
-    // two million queries: two lists of kListCap were as large)
-    if (lazy && tc_column_groups(k) == 4 &&
+    // two million queries: two lists of kListCap hold as much, which is what
+    // eight epilogue warps, and the fp32 screen of rows under 16 features, take)
+    if ((lazy || (tc && ix.d < 16)) && tc_column_groups(k) == 4 &&
         (size_t)S_lists * m_pad * kListCap * sizeof(int2) > ((size_t)32 << 30))
       so.cap = kListCap / 2;
     so.m_pad = (int)m_pad;
     ws.reserve(&so.lists, (size_t)S_lists * m_pad * so.cap);
     ws.reserve(&so.counts, (size_t)S_lists * m_pad);
     if (!lazy) ws.reserve(&so.kth, (size_t)S_lists * m_pad * k);
-    if (seed) {
-      ws.reserve(&home, (size_t)m_tiles);
-      ws.reserve(&seed_counts, (size_t)seed_groups * m_pad);
-      ws.reserve(&seed_kth, (size_t)seed_groups * m_pad * seed_k);
+    if (seed) ws.reserve(&home, (size_t)m_tiles);
+    if (seed || spread) {
+      const size_t seed_lists = (size_t)(spread ? spread_S : 1) * seed_groups;
+      ws.reserve(&seed_counts, seed_lists * m_pad);
+      ws.reserve(&seed_kth, seed_lists * m_pad * seed_k);
     }
     ws.reserve(&fb_list, (size_t)m);
     if ((rc = ws.place(st, fr))) return rc;
@@ -800,9 +817,10 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
       // k = 50: list entries 88M -> 37M, screen 5.71 -> 2.38 ms (1.79 with
       // sixteen epilogue warps).  Filling the lazy tracker's own lists in the
       // pass instead cost 2.3 ms, the pass itself 0.45.
-      if (seed) {
-        launch_home_tiles(perm, key, m, ix.group_start, (int)n_tiles, kSeedTiles, home,
-                          (int)m_tiles, st);
+      if (seed || spread) {
+        if (seed)
+          launch_home_tiles(perm, key, m, ix.group_start, (int)n_tiles, kSeedTiles, home,
+                            (int)m_tiles, st);
         SinkArgs sb = sa;
         sb.out.cap = 0;  // the trackers only: no list entry is written
         sb.out.counts = seed_counts;
@@ -810,12 +828,14 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
         sb.k = seed_k;
         if (lazy) sb.shared_kth = nullptr;  // a group's 16th value is not the query's k-th
         // status[7] (zeroed above) counts this pass's claimed units
-        int lr = launch_screen_tc(&ix, &tmap_a, m, m_pad, exclude_self, q_offset, 1, qp.E,
-                                  kSinkKnn, sb, status, st, perm, status + 7, tf32, home,
-                                  kSeedTiles);
+        int lr = launch_screen_tc(&ix, &tmap_a, m, m_pad, exclude_self, q_offset,
+                                  spread ? spread_S : 1, qp.E, kSinkKnn, sb, status, st, perm,
+                                  status + 7, tf32, home, spread ? spread_window : kSeedTiles);
         if (lr) return fail(B2K_ECUDA, "tcgen05 seeding screen launch failed: %s",
                             cudaGetErrorString((cudaError_t)lr));
-        if (lazy && seed_groups * seed_k >= k)
+        if (spread)
+          launch_seed_kth_spread(seed_kth, spread_S * seed_groups, m, m_pad, k, shared_kth, st);
+        else if (lazy && seed_groups * seed_k >= k)
           launch_seed_kth(seed_kth, seed_groups, seed_k, m, m_pad, k, shared_kth, st);
         if (stats) cudaEventRecord(ev[4], st);
         seeded = true;

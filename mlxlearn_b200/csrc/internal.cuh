@@ -205,6 +205,8 @@ struct SinkArgs;
 // tf32: the kind::tf32 form over the index's tf32 operand (kNN sinks only).
 // home (with S = 1): query tile t scans only reference tiles
 // [home[t], home[t] + home_tiles) -- the seeding pass of grouped rows.
+// home_tiles without home: split s scans only the home_tiles tiles from
+// s * (tiles / S) on -- the spread seeding pass.
 int launch_screen_tc(Index* ix, const CUtensorMap* tmap_a, int64_t m, int64_t m_pad,
                      int exclude_self, int64_t q_offset, int S, const float* E, int sink_kind,
                      const SinkArgs& sa, int* status, cudaStream_t st,
@@ -259,6 +261,12 @@ void launch_home_tiles(const int* perm, const int* key, int64_t m, const int* gr
 // lists of kl, kth [groups][m_pad][kl] (unchanged when fewer than k are finite)
 void launch_seed_kth(const float* kth, int groups, int kl, int64_t m, int64_t m_pad, int k,
                      uint32_t* shared_kth, cudaStream_t st);
+
+// No smaller than that value, for the many lists of a spread pass (kl = 16,
+// k <= 64): a warp per query, exact while no lane's lists hold more than 16 of
+// the k smallest.
+void launch_seed_kth_spread(const float* kth, int lists, int64_t m, int64_t m_pad, int k,
+                            uint32_t* shared_kth, cudaStream_t st);
 
 // The batched form: problem p owns global rows [row_start[p], row_start[p + 1]);
 // m = 0 leaves a problem's words alone.

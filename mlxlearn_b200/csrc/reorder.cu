@@ -424,6 +424,57 @@ __global__ void seed_kth_kernel(const float* __restrict__ kth, int G, int kl, in
   if (r < m) seed_kth_row(kth, G, kl, r, m_pad, k, shared_kth);
 }
 
+// A warp per query: each lane merges its lists (lane, lane + 32, ...) into the 16
+// smallest, then the k-th smallest of those by k warp minima.  What a lane drops
+// can only make the result larger, which a threshold may be.  Bound by latency:
+// a few loads and k reductions; a thread per query walking the heads of 32 or
+// more lists would take k times as many dependent steps.
+__global__ void seed_kth_spread_kernel(const float* __restrict__ kth, int G, int64_t m,
+                                       int64_t m_pad, int k, uint32_t* __restrict__ shared_kth) {
+  const int lane = threadIdx.x & 31;
+  const int64_t r = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+  if (r >= m) return;
+  constexpr int kL = 16;
+  const uint32_t none = float_key(INFINITY);
+  uint32_t key[kL];
+#pragma unroll
+  for (int j = 0; j < kL; ++j) key[j] = none;
+  for (int g = lane; g < G; g += 32) {
+    const float4* src = reinterpret_cast<const float4*>(kth + ((size_t)g * m_pad + r) * kL);
+    // both ascend: the 16 smaller of (key[j], list[15 - j]) are the smallest 16,
+    // a bitonic sequence
+#pragma unroll
+    for (int j = 0; j < kL; j += 4) {
+      const float4 v = src[j / 4];
+      key[kL - 1 - j] = min(key[kL - 1 - j], float_key(v.x));
+      key[kL - 2 - j] = min(key[kL - 2 - j], float_key(v.y));
+      key[kL - 3 - j] = min(key[kL - 3 - j], float_key(v.z));
+      key[kL - 4 - j] = min(key[kL - 4 - j], float_key(v.w));
+    }
+#pragma unroll
+    for (int h = kL / 2; h > 0; h >>= 1)
+#pragma unroll
+      for (int j = 0; j < kL; ++j)
+        if (!(j & h)) {
+          const uint32_t a = key[j], b = key[j + h];
+          key[j] = min(a, b);
+          key[j + h] = max(a, b);
+        }
+  }
+  __syncwarp();
+  uint32_t best = none;
+  for (int t = 0; t < k; ++t) {
+    best = __reduce_min_sync(0xffffffffu, key[0]);
+    const unsigned who = __ballot_sync(0xffffffffu, key[0] == best);
+    if (lane == __ffs(who) - 1) {
+#pragma unroll
+      for (int j = 0; j + 1 < kL; ++j) key[j] = key[j + 1];
+      key[kL - 1] = none;
+    }
+  }
+  if (lane == 0 && best < none) shared_kth[r] = best;
+}
+
 __global__ void seed_kth_batch_kernel(const SeedProblem* __restrict__ tab,
                                       const int64_t* __restrict__ row_start, int P,
                                       int64_t total) {
@@ -458,6 +509,13 @@ void launch_seed_kth(const float* kth, int groups, int kl, int64_t m, int64_t m_
   if (m <= 0) return;
   seed_kth_kernel<<<(unsigned)((m + 127) / 128), 128, 0, st>>>(kth, groups, kl, m, m_pad, k,
                                                                shared_kth);
+}
+
+void launch_seed_kth_spread(const float* kth, int lists, int64_t m, int64_t m_pad, int k,
+                            uint32_t* shared_kth, cudaStream_t st) {
+  if (m <= 0) return;
+  seed_kth_spread_kernel<<<(unsigned)((m + 3) / 4), 128, 0, st>>>(kth, lists, m, m_pad, k,
+                                                                  shared_kth);
 }
 
 void launch_seed_kth_batch(const SeedProblem* tab, const int64_t* row_start, int P,

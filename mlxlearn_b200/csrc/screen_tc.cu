@@ -80,6 +80,7 @@ struct TcParams {
   int* status;
   int* unit_counter;         // units claimed dynamically (or null: round-robin / per-CTA lists)
   const int* home;           // single problem, seeding pass: tile t's window starts at home[t]
+  int split_step;            // single problem: first tile of split s = s * split_step
   int n_items;               // batched, claimed: items in the list
   TcProblem one;             // single problem
 };
@@ -181,7 +182,7 @@ struct UnitCursor {
       const int s = w / p.m_tiles;
       x.pr = &p.one;
       x.t = w % p.m_tiles;
-      x.j0 = p.home ? p.home[x.t] : s * p.one.tiles_per_split;
+      x.j0 = p.home ? p.home[x.t] : s * p.split_step;
       x.j1 = min(x.j0 + p.one.tiles_per_split, p.one.n_tiles);
       x.slot = s;
     }
@@ -722,6 +723,9 @@ int launch_screen_tc(Index* ix, const CUtensorMap* tmap_a, int64_t m, int64_t m_
                      int* unit_counter, bool tf32, const int* home, int home_tiles) {
   if (tf32 && sink_kind != kSinkKnn) return (int)cudaErrorInvalidValue;
   if (home && (S != 1 || home_tiles <= 0)) return (int)cudaErrorInvalidValue;
+  // (spread windows must not share a tile: its columns would count twice)
+  if (!home && home_tiles > 0 && (int64_t)S * home_tiles > ix->n_pad_tc / kTcBN)
+    return (int)cudaErrorInvalidValue;
   TcParams p{};
   p.unit_counter = unit_counter;
   p.home = home;
@@ -729,7 +733,8 @@ int launch_screen_tc(Index* ix, const CUtensorMap* tmap_a, int64_t m, int64_t m_
   one.m = (int)m;
   one.KB = tf32 ? ix->dpt / kTcBKf : ix->dp / kTcBK;
   one.n_tiles = (int)(ix->n_pad_tc / kTcBN);
-  one.tiles_per_split = home ? home_tiles : (one.n_tiles + S - 1) / S;
+  one.tiles_per_split = home_tiles > 0 ? home_tiles : (one.n_tiles + S - 1) / S;
+  p.split_step = home_tiles > 0 ? one.n_tiles / S : one.tiles_per_split;
   one.exclude_self = exclude_self;
   one.q_offset = q_offset;
   one.E = E;
@@ -795,6 +800,7 @@ int launch_screen_tc_u8(Index* ix, const CUtensorMap* tmap_a, int64_t m, int64_t
   one.KB = ix->dpu / kTcBKu;
   one.n_tiles = (int)(ix->n_pad_tc / kTcBN);
   one.tiles_per_split = (one.n_tiles + S - 1) / S;
+  p.split_step = one.tiles_per_split;
   one.exclude_self = exclude_self;
   one.q_offset = q_offset;
   one.nxu = ix->nxu;  // training order: the self column is the training row

@@ -49,3 +49,25 @@ def test_many_lists(m, k):
     ed, ei = oracle.knn(X, Q, k)
     assert np.array_equal(idx, ei)
     assert np.array_equal(dist, ed)
+
+
+# seeding windows spread over the rows: 4 windows of 8 or 9 tiles, one window a
+# tile with a ragged end, two tiles a window; 64 is the widest k
+@pytest.mark.parametrize("n,m", [(2048, 5), (2049, 300), (20011, 2047), (100003, 1500)])
+@pytest.mark.parametrize("d,k", [(5, 17), (20, 64)])
+def test_spread_seeding(n, m, d, k):
+    X, Q = _rows(n, d, n + m, 0), _rows(m, d, n + d, 50)
+    X[100:140] = X[:40]
+    Q[:5] = X[:5]
+    dist, idx = build_index(X).query(Q, k)
+    ed, ei = oracle.knn(X, Q, k)
+    assert np.array_equal(idx, ei)
+    assert np.array_equal(dist, ed)
+
+
+def test_spread_seeding_self():
+    X = _rows(6001, 12, 3, 30)
+    dist, idx = build_index(X).query(X, 30, exclude_self=True)
+    ed, ei = oracle.knn(X, X, 30, exclude_self=True)
+    assert np.array_equal(idx, ei)
+    assert np.array_equal(dist, ed)

@@ -403,6 +403,15 @@ __device__ __forceinline__ int refine_candidates(const CertifyArgs& a, int64_t r
   return C;
 }
 
+// The k-th smallest of a full candidate buffer of screen values; `scratch` holds
+// 256 words.
+constexpr int kTighten = 3;  // gathers again with a bound from the buffer, at most
+__device__ __forceinline__ float listed_kth(const float* cv, int k, void* scratch, int lane) {
+  auto value_key = [&](int c) { return float_key(cv[c]); };
+  unsigned* hist = static_cast<unsigned*>(scratch);
+  return key_float(warp_radix_kth(value_key, kCertifyCap, k, hist, lane));
+}
+
 // One query row of one problem, by one warp; `wbase` is the warp's shared
 // memory (kCertWarpBytes).
 // GATHERED: (ci, cv) already hold the `gathered` >= k entries within 2E of the
@@ -533,7 +542,20 @@ __device__ __forceinline__ void certify_row(const CertifyArgs& a, int64_t row, u
   if constexpr (GATHERED) {
     C = gathered;
   } else if (bound_key != 0xffffffffu) {
-    C = gather(__fadd_ru(key_float(bound_key), E2));
+    float limit = __fadd_ru(key_float(bound_key), E2);
+    C = gather(limit);
+    // More than fit: the k-th smallest of those that did bounds V_k as well
+    // (a shared word set by short lists, or by a pass over other regions, can be
+    // loose).  30,000 x 100, 30 queries, k = 15 (236 lists of 127 columns):
+    // 391 us falling through to the lists' own k-th values, 0.50 -> 0.16 ms a call.
+    for (int i = 0; i < kTighten && C > kCertifyCap; ++i) {
+      __syncwarp();
+      const float l = __fadd_ru(listed_kth(cv, k, cs, lane), E2);
+      __syncwarp();
+      if (!(l < limit)) break;
+      limit = l;
+      C = gather(limit);
+    }
     cut = C >= k && C <= kCertifyCap;
     if (!cut) C = -1;
   }
@@ -756,6 +778,7 @@ __global__ void __launch_bounds__(kWideThreads)
   extern __shared__ uint8_t smem[];
   __shared__ unsigned s_sum[kWideThreads / 32];
   __shared__ int s_count;
+  __shared__ float s_limit;
   int* ci = reinterpret_cast<int*>(smem);
   float* cv = reinterpret_cast<float*>(ci + kCertifyCap);
   unsigned* off = reinterpret_cast<unsigned*>(smem + kCertWarpBytes) - kFlatLists;  // certify_row's hist
@@ -786,41 +809,57 @@ __global__ void __launch_bounds__(kWideThreads)
     }
     if (tid < S) off[tid] = before + incl - (unsigned)c;
     __syncthreads();
-    const float limit = __fadd_ru(key_float(key), __fmul_ru(2.0f, a.E[row]));
+    const float E2 = __fmul_ru(2.0f, a.E[row]);
+    float limit = __fadd_ru(key_float(key), E2);
     constexpr int kAhead = 4;
-    for (unsigned base = 0; base < entries; base += kWideThreads * kAhead) {
-      int2 e[kAhead];
-      bool in[kAhead];
-#pragma unroll
-      for (int u = 0; u < kAhead; ++u) {
-        const unsigned i = base + kWideThreads * u + tid;
-        in[u] = i < entries;
-        e[u] = make_int2(0, 0);
-        if (in[u]) {
-          int lo = 0, hi = S - 1;  // the last list whose offset is <= i
-          while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (off[mid] <= i)
-              lo = mid;
-            else
-              hi = mid - 1;
+    for (int again = 0;; ++again) {
+      for (unsigned base = 0; base < entries; base += kWideThreads * kAhead) {
+        int2 e[kAhead];
+        bool in[kAhead];
+  #pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          const unsigned i = base + kWideThreads * u + tid;
+          in[u] = i < entries;
+          e[u] = make_int2(0, 0);
+          if (in[u]) {
+            int lo = 0, hi = S - 1;  // the last list whose offset is <= i
+            while (lo < hi) {
+              const int mid = (lo + hi + 1) >> 1;
+              if (off[mid] <= i)
+                lo = mid;
+              else
+                hi = mid - 1;
+            }
+            e[u] = so.lists[((size_t)lo * so.m_pad + row) * so.cap + (i - off[lo])];
           }
-          e[u] = so.lists[((size_t)lo * so.m_pad + row) * so.cap + (i - off[lo])];
+        }
+  #pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          const float v = __int_as_float(e[u].x);
+          const bool pass = in[u] && v <= limit;
+          const unsigned bal = __ballot_sync(0xffffffffu, pass);
+          int pos = 0;
+          if (lane == 0 && bal) pos = atomicAdd(&s_count, __popc(bal));
+          pos = __shfl_sync(0xffffffffu, pos, 0) + __popc(bal & ((1u << lane) - 1));
+          if (pass && pos < kCertifyCap) {
+            ci[pos] = e[u].y;
+            cv[pos] = v;
+          }
         }
       }
-#pragma unroll
-      for (int u = 0; u < kAhead; ++u) {
-        const float v = __int_as_float(e[u].x);
-        const bool pass = in[u] && v <= limit;
-        const unsigned bal = __ballot_sync(0xffffffffu, pass);
-        int pos = 0;
-        if (lane == 0 && bal) pos = atomicAdd(&s_count, __popc(bal));
-        pos = __shfl_sync(0xffffffffu, pos, 0) + __popc(bal & ((1u << lane) - 1));
-        if (pass && pos < kCertifyCap) {
-          ci[pos] = e[u].y;
-          cv[pos] = v;
-        }
+      __syncthreads();
+      if (s_count <= kCertifyCap || again == kTighten) break;  // block-uniform
+      // more than fit: a tighter limit from those that did, as in certify_row
+      if (w == 0) {
+        const float l = listed_kth(cv, a.k, cv + kCertifyCap, lane);
+        if (lane == 0) s_limit = __fadd_ru(l, E2);
       }
+      __syncthreads();
+      const float l = s_limit;
+      if (!(l < limit)) break;
+      limit = l;
+      if (tid == 0) s_count = 0;
+      __syncthreads();
     }
   }
   __syncthreads();

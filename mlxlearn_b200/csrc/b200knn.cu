@@ -708,8 +708,15 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
     if (grouped && (rc = ensure_pivots(ix))) return rc;
     const int64_t m_tiles = m_pad / kTcBM;
     const int kSeedTiles = seed_tiles();
+    // A query tile's home window is one unit of 16 tiles, so below a unit an SM
+    // the pass is one long wave, and the main screen of a small call is as short.
+    // Register trackers (call with the pass / without): 8,192 x 64, 6,000 queries,
+    // k = 5: 231 / 198 us; 120,000 x 15, 6,000: 426 / 393; 30,000 x 64, 20,000: 535
+    // / 525 and 50,000: 974 / 1,040; 120,000 x 64, 20,000: 966 / 1,057; 500,000 x 15,
+    // 20,000, k = 15: 3,576 / 3,726.  A lazy tracker needs some threshold always.
     const bool seed = tc && grouped && ix.group_start && n_tiles >= 2 * kSeedTiles &&
-                      seed_enabled();
+                      seed_enabled() &&
+                      (lazy || (m_tiles >= sms && m_tiles * n_tiles >= 256 * (int64_t)sms));
     const int seed_k = lazy ? 16 : k, seed_groups = tc ? tc_column_groups(seed_k) : 0;
     // Lazy lists without grouped queries (m < 2048 or few rows) are seeded from
     // windows spread over the rows: an eighth of the tiles, 4 to 64 (128 where the

@@ -352,14 +352,14 @@ int knn_backward(const float* Q, int64_t m, const float* X, int64_t n, int d, in
   if (dX && n > 0) {
     const int64_t mk = m * (int64_t)k;
     int* counts = workspace;           // [n]
-    int* offsets = counts + n;         // [n + 1]
-    int* cursor = offsets + n + 1;     // [n]
-    int* order = cursor + n;           // [mk]
+    int* cursor = counts + n;          // [n]
+    int* big_count = cursor + n;       // zeroed with the two before it
+    int* offsets = big_count + 1;      // [n + 1]
+    int* order = offsets + n + 1;      // [mk]
     int* sums = order + mk;            // [nb + 1] block sums of the scan
     const int nb = (int)((n + kScanBlock - 1) / kScanBlock);
     int* sorted = sums + nb + 1;       // [mk] buckets in ascending flat order
-    cudaMemsetAsync(counts, 0, (size_t)n * sizeof(int), st);
-    cudaMemsetAsync(cursor, 0, (size_t)n * sizeof(int), st);
+    cudaMemsetAsync(counts, 0, ((size_t)2 * n + 1) * sizeof(int), st);
     if (mk > 0)
       bucket_count_kernel<<<(unsigned)((mk + 255) / 256), 256, 0, st>>>(idx, mk, counts);
     scan_sums_kernel<<<nb, kScanThreads, 0, st>>>(counts, n, sums);
@@ -372,23 +372,23 @@ int knn_backward(const float* Q, int64_t m, const float* X, int64_t n, int d, in
       grad_x_narrow_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
           Q, X, G, E, offsets, order, n, d, k, squared, dX);
     else {
-      // the bucket cursors and counts are free by now: the big rows and their number
-      int* big = cursor;
-      int* big_count = counts;
-      cudaMemsetAsync(big_count, 0, sizeof(int), st);
+      int* big = cursor;  // (free by now)
       grad_x_kernel<<<(unsigned)((n + warps - 1) / warps), warps * 32, 0, st>>>(
           Q, X, G, E, offsets, order, sorted, n, d, k, squared, big, big_count, dX);
       int dev = 0;
       cudaGetDevice(&dev);
-      grad_x_big_kernel<<<4 * num_sms(dev), kBigThreads, 0, st>>>(
-          Q, X, G, E, offsets, order, sorted, d, k, squared, big, big_count, dX);
+      // (no more big buckets than their picks allow)
+      const int64_t most = std::min<int64_t>(4 * num_sms(dev), mk / kBigBucket);
+      if (most > 0)
+        grad_x_big_kernel<<<(unsigned)most, kBigThreads, 0, st>>>(
+            Q, X, G, E, offsets, order, sorted, d, k, squared, big, big_count, dX);
     }
   }
   return (int)cudaGetLastError();
 }
 
 size_t knn_backward_workspace_ints(int64_t m, int64_t n, int k) {
-  return (size_t)(3 * n + 1) + 2 * (size_t)m * k + (size_t)((n + kScanBlock - 1) / kScanBlock) +
+  return (size_t)(3 * n + 2) + 2 * (size_t)m * k + (size_t)((n + kScanBlock - 1) / kScanBlock) +
          1;
 }
 

@@ -604,16 +604,17 @@ extern "C" B2K_API int b2k_knn_segments(const float* dQ, const float* dX, int32_
     put(dblocks, blocks.data(), blk_b);
     put(tab, ex.data(), tab_b);
     if ((e = cudaMemcpyAsync(base, up.data(), up.size(), cudaMemcpyHostToDevice, st)) ||
-        (e = cudaMemsetAsync(flags, 0, 16 * sizeof(int), st)) ||
-        (e = cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), st))) {
+        (e = cudaMemsetAsync(flags, 0, base + bytes - reinterpret_cast<unsigned char*>(flags),
+                             st))) {  // flags and counters
       rc = seg_fail(B2K_ECUDA, "b2k_knn_segments: copy to the device failed");
       break;
     }
     const int64_t nq = rows * d, nx = x_offsets[P] * d;
     seg_range_kernel<<<(unsigned)std::min<int64_t>((nq + 255) / 256 + 1, 1024), 256, 0, st>>>(
         dQ, nq, flags);
-    seg_range_kernel<<<(unsigned)std::min<int64_t>((nx + 255) / 256 + 1, 1024), 256, 0, st>>>(
-        dX, nx, flags);
+    if (dX != dQ || nx != nq)
+      seg_range_kernel<<<(unsigned)std::min<int64_t>((nx + 255) / 256 + 1, 1024), 256, 0, st>>>(
+          dX, nx, flags);
     SegArgs a{};
     a.Q = dQ;
     a.X = dX;

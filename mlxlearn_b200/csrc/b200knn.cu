@@ -14,6 +14,7 @@
 #include <climits>
 #include <cstdarg>
 #include <cmath>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -55,7 +56,7 @@ static int fail(int code, const char* fmt, ...) {
                   #call, cudaGetErrorString(e_), __FILE__, __LINE__);                       \
   } while (0)
 
-// Host-side fault injection for failure-path tests (B2K_FAULT=alloc|launch|timeout).
+// Host-side fault injection for failure-path tests (B2K_FAULT=alloc|alloc:N|launch|timeout).
 static int fault_mode() {
   const char* f = getenv("B2K_FAULT");
   if (!f || !*f) return 0;
@@ -63,6 +64,19 @@ static int fault_mode() {
   if (!strcmp(f, "launch")) return 2;
   if (!strcmp(f, "timeout")) return 3;
   return 0;
+}
+
+// Whether this device allocation is to fail: every one under B2K_FAULT=alloc,
+// the N-th since the variable was set under alloc:N (counted while it is set).
+static bool inject_alloc_failure() {
+  static std::atomic<long> seen{0};
+  const char* f = getenv("B2K_FAULT");
+  if (!f || strncmp(f, "alloc", 5)) {
+    seen.store(0, std::memory_order_relaxed);
+    return false;
+  }
+  if (!f[5]) return true;
+  return f[5] == ':' && seen.fetch_add(1) + 1 == atol(f + 6);
 }
 
 uint32_t device_spin_limit() {
@@ -170,7 +184,8 @@ static int check_device(int device) {
 
 template <typename T>
 static int dalloc(T** p, size_t count, cudaStream_t st) {
-  if (fault_mode() == 1) return fail(B2K_ENOMEM, "injected allocation failure (B2K_FAULT=alloc)");
+  if (inject_alloc_failure())
+    return fail(B2K_ENOMEM, "injected allocation failure (B2K_FAULT=alloc)");
   *p = nullptr;
   if (count == 0) count = 1;
   cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(p), count * sizeof(T), st);
@@ -190,6 +205,8 @@ static int dalloc(T** p, size_t count, cudaStream_t st) {
 constexpr size_t kPoolAlloc = (size_t)32 << 20;
 template <typename T>
 static int ialloc(Index& ix, T** p, size_t count) {
+  if (inject_alloc_failure())
+    return fail(B2K_ENOMEM, "injected allocation failure (B2K_FAULT=alloc)");
   const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
   const bool pooled = bytes <= kPoolAlloc;
   void* v = nullptr;
@@ -284,19 +301,27 @@ static int finish_index(Index& ix, cudaStream_t st) {
   return B2K_OK;
 }
 
-// Pivots for query grouping and row grouping (the caller holds ix.mu).
+// Pivots for query grouping and row grouping (the caller holds ix.mu).  Set
+// together and last: ix.pivots tells that all of them are built, so a failed
+// allocation or launch leaves the index without pivots and a later call starts
+// over.
 static int make_pivots(Index& ix) {
   if (ix.pivots) return B2K_OK;
   int rc;
-  ix.n_pivots = pivot_count(ix.n);
-  if ((rc = ialloc(ix, &ix.pivots, (size_t)ix.n_pivots * ix.d))) return rc;
-  if ((rc = ialloc(ix, &ix.pivot_norms, (size_t)ix.n_pivots))) return rc;
-  ix.pivot_dpa = pivot_dims_padded(ix.d);
-  if ((rc = ialloc(ix, &ix.pivots_h, (size_t)pivot_rows_padded(ix.n_pivots) * ix.pivot_dpa)))
-    return rc;
-  launch_pivots(&ix, ix.stream);
+  const int P = pivot_count(ix.n), dpa = pivot_dims_padded(ix.d);
+  float *pivots = nullptr, *norms = nullptr;
+  uint16_t* rows = nullptr;
+  if ((rc = ialloc(ix, &pivots, (size_t)P * ix.d))) return rc;
+  if ((rc = ialloc(ix, &norms, (size_t)P))) return rc;
+  if ((rc = ialloc(ix, &rows, (size_t)pivot_rows_padded(P) * dpa))) return rc;
+  launch_pivots(&ix, P, dpa, pivots, norms, rows, ix.stream);
   B2K_CUDA(cudaGetLastError());
   B2K_CUDA(cudaStreamSynchronize(ix.stream));
+  ix.n_pivots = P;
+  ix.pivot_dpa = dpa;
+  ix.pivot_norms = norms;
+  ix.pivots_h = rows;
+  ix.pivots = pivots;
   return B2K_OK;
 }
 

@@ -234,7 +234,10 @@ int simt_column_groups(int sink_kind, bool noalloc = false);
 int pivot_count(int64_t n);
 int pivot_rows_padded(int P);  // pivots padded to the assignment's tile
 int pivot_dims_padded(int d);  // features padded to its chunk
-void launch_pivots(Index* ix, cudaStream_t st);
+// P = pivot_count(n) pivots of the index into [P, d], their norms [P] and the
+// bf16 operand [pivot_rows_padded(P), dpa]
+void launch_pivots(const Index* ix, int P, int dpa, float* pivots, float* norms,
+                   uint16_t* pivots_h, cudaStream_t st);
 // perm[i] = original row of sorted position i; Qp = Q[perm]; hist zeroed by the caller
 // best64: assign_scratch(ix, m) words, or null when that is 0
 size_t assign_scratch(const Index* ix, int64_t m);

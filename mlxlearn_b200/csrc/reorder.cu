@@ -548,13 +548,12 @@ int pivot_count(int64_t n) {
 int pivot_rows_padded(int P) { return (P + kMmaP - 1) / kMmaP * kMmaP; }
 int pivot_dims_padded(int d) { return (d + kMmaK - 1) / kMmaK * kMmaK; }
 
-void launch_pivots(Index* ix, cudaStream_t st) {
-  pivot_rows_kernel<<<ix->n_pivots, 32, 0, st>>>(ix->X, ix->n, ix->d, ix->n_pivots, ix->center,
-                                                 ix->pivots, ix->pivot_norms);
-  const int64_t total = (int64_t)pivot_rows_padded(ix->n_pivots) * ix->pivot_dpa;
+void launch_pivots(const Index* ix, int P, int dpa, float* pivots, float* norms,
+                   uint16_t* pivots_h, cudaStream_t st) {
+  pivot_rows_kernel<<<P, 32, 0, st>>>(ix->X, ix->n, ix->d, P, ix->center, pivots, norms);
+  const int64_t total = (int64_t)pivot_rows_padded(P) * dpa;
   pivots_bf16_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(
-      ix->pivots, ix->n_pivots, ix->d, pivot_rows_padded(ix->n_pivots), ix->pivot_dpa,
-      ix->pivots_h);
+      pivots, P, ix->d, pivot_rows_padded(P), dpa, pivots_h);
 }
 
 // Pivot tiles a block takes: all while the query blocks fill the GPU, else as

@@ -289,6 +289,24 @@ static int finish_index(Index& ix, cudaStream_t st) {
   B2K_CUDA(cudaMemsetAsync(ix.stats_dev, 0, kStatsLen * sizeof(float), st));
   launch_prep_index(&ix, st);
   B2K_CUDA(cudaGetLastError());
+  // narrow rows: the sample that chooses their screen (NarrowProfile)
+  const bool narrow = ix.d >= kTcMinD && ix.d < kTcAlwaysD && ix.n >= kTcMinN;
+  struct Sample {
+    double norms[kProfileSamples];
+    int hist[kProfileSamples * kProfileBins];
+  };
+  StreamFree fr{st, {}};
+  std::vector<Sample> sample(narrow ? 1 : 0);
+  const int rows = profile_rows(ix.n);
+  if (narrow) {
+    Sample* dev = nullptr;
+    if (const int rc = dalloc(&dev, 1, st)) return rc;
+    fr.keep(dev);
+    B2K_CUDA(cudaMemsetAsync(dev, 0, sizeof(Sample), st));
+    launch_narrow_profile(&ix, rows, dev->hist, dev->norms, st);
+    B2K_CUDA(cudaGetLastError());
+    B2K_CUDA(cudaMemcpyAsync(sample.data(), dev, sizeof(Sample), cudaMemcpyDeviceToHost, st));
+  }
   float stats[kStatsLen];
   B2K_CUDA(cudaMemcpyAsync(stats, ix.stats_dev, sizeof(stats), cudaMemcpyDeviceToHost, st));
   B2K_CUDA(cudaStreamSynchronize(st));
@@ -298,7 +316,109 @@ static int finish_index(Index& ix, cudaStream_t st) {
   int bad;
   memcpy(&bad, &stats[2], 4);
   ix.range_ok = bad == 0;
+  // (below 2^-80 the bins would leave the float range: such rows take the fp32 screen)
+  if (narrow && ix.range_ok && ix.nx_max > 0x1p-80f) {
+    NarrowProfile& p = ix.profile;
+    std::nth_element(sample[0].norms, sample[0].norms + kProfileSamples / 2,
+                     sample[0].norms + kProfileSamples);
+    p.rms = (float)std::sqrt(sample[0].norms[kProfileSamples / 2]);
+    p.base = profile_base(ix.nx_max);
+    p.cum.assign((size_t)kProfileSamples * (kProfileBins + 1), 0);
+    for (int s = 0; s < kProfileSamples; ++s) {
+      int* cum = p.cum.data() + (size_t)s * (kProfileBins + 1);
+      for (int b = 0; b < kProfileBins; ++b)
+        cum[b + 1] = cum[b] + sample[0].hist[s * kProfileBins + b];
+    }
+    p.rows = rows;
+  }
   return B2K_OK;
+}
+
+// ------------------------------------------- which screen narrow rows take
+// Lower edge of bin b of a profile (the first bin reaches down to zero).
+static double profile_edge(const NarrowProfile& p, int b) {
+  if (b <= 0) return 0.0;
+  const uint32_t bits = (uint32_t)(b + p.base) << 21;
+  float v;
+  memcpy(&v, &bits, sizeof(v));
+  return v;
+}
+
+// Rows of sample s within squared distance t (interpolated in t's bin).
+static double profile_within(const NarrowProfile& p, int s, double t) {
+  const int* cum = p.cum.data() + (size_t)s * (kProfileBins + 1);
+  const float tf = (float)t;
+  uint32_t bits;
+  memcpy(&bits, &tf, sizeof(bits));
+  const int b = std::max((int)(bits >> 21) - p.base, 0);
+  if (b >= kProfileBins) return cum[kProfileBins];
+  const double lo = profile_edge(p, b), hi = profile_edge(p, b + 1);
+  return cum[b] + (cum[b + 1] - cum[b]) * std::min(1.0, (t - lo) / (hi - lo));
+}
+
+// Squared distance within which sample s has `rows` rows.
+static double profile_radius2(const NarrowProfile& p, int s, double rows) {
+  const int* cum = p.cum.data() + (size_t)s * (kProfileBins + 1);
+  const int b = (int)(std::lower_bound(cum + 1, cum + kProfileBins, rows) - cum) - 1;
+  const double lo = profile_edge(p, b), hi = profile_edge(p, b + 1);
+  const int in = cum[b + 1] - cum[b];
+  return in > 0 ? lo + (hi - lo) * std::min(1.0, std::max(0.0, (rows - cum[b]) / in)) : hi;
+}
+
+// The certified error of the tensor-core screen for a query at the samples'
+// median distance from the centre (prep.cu derives it).
+static double profile_error(const Index& ix) {
+  const double g = (double)(round_up(ix.d, kTcBK) + kTcAug + 16) * 0x1p-20;
+  return 1.02 * g * (2.0 * ix.profile.rms * ix.xn_max + ix.nx_max);
+}
+
+// Whether AUTO sends m queries to the tensor cores.  Under 16 features by the
+// band the sample predicts: rows within 2E of the k-th distance.
+// * Large calls: while a quarter of the samples at most hold more than the 1,024
+//   that certify takes.  (Tensor cores / fp32 screen by that share, 200,003 rows,
+//   50,021 queries: 0.31 10.9 / 17.4 ms at k = 5, 19.3 / 18.5 at k = 15; 0.61
+//   15.1 / 16.9 at k = 5 and 51 / 31.5 at k = 50; 0.77 22.5 / 17.5; 0.95 60 / 17.)
+// * Small calls (the fp32 screen takes under 0.5 ms) pay every listed row with
+//   latency and a second pass whole: 10,000 x 8, 2,000 queries, k = 5: 20 band
+//   rows 0.138 / 0.145 ms, 88 0.157 / 0.141, 502 0.265 / 0.146; k = 50: 106
+//   0.187 / 0.369.  20,000 x 5, 100 queries, k = 5: 110 0.137 / 0.098.
+// The predicted share agrees with the measured one to a few percent over normal,
+// uniform, heavy-tailed and clustered rows and one far row or column.
+static bool knn_on_tensor_cores(const Index& ix, int64_t m, int k) {
+  if (ix.d < kTcMinD || ix.n < kTcMinN) return false;
+  if (ix.d >= kTcAlwaysD) return true;
+  const NarrowProfile& p = ix.profile;
+  if (!p.rows) return false;
+  const bool small = m * ix.n < ((int64_t)1 << 28);
+  const double limit = small ? 2.0 * k + 32.0 : 1024.0;
+  const double scale = (double)ix.n / p.rows;
+  const double kth = std::max(1.0, k / scale), band = 2.0 * profile_error(ix);
+  int wide = 0;
+  for (int s = 0; s < kProfileSamples; ++s) {
+    const double t = profile_radius2(p, s, kth);
+    if ((profile_within(p, s, t + band) - kth) * scale + k > limit) ++wide;
+  }
+  return wide * 4 <= kProfileSamples;
+}
+
+// Whether the radius search sends its queries to the tensor cores: as
+// above, by the rows in (R2, R2 + 2E] a query.  Every one is a candidate (12 bytes
+// of scratch and an exact test), so they are kept below 1,024, or below the
+// answer's own size: 200,003 x 8, 20,000 queries, 90 neighbours: 421 candidates 1.4
+// / 13.1 ms, 2,082 2.0, 38,007 6.9 ms and 9 GB, where the fp32 screen has 93.
+static bool radius_on_tensor_cores(const Index& ix, double R2) {
+  if (ix.d < kTcMinD || ix.n < kTcMinN) return false;
+  if (ix.d >= kTcAlwaysD) return true;
+  const NarrowProfile& p = ix.profile;
+  if (!p.rows) return false;
+  const double band = 2.0 * profile_error(ix);
+  double inside = 0, wide = 0;
+  for (int s = 0; s < kProfileSamples; ++s) {
+    inside += profile_within(p, s, R2);
+    wide += profile_within(p, s, R2 + band);
+  }
+  const double scale = (double)ix.n / p.rows / kProfileSamples;
+  return (wide - inside) * scale <= std::max(1024.0, inside * scale);
 }
 
 // Pivots for query grouping and row grouping (the caller holds ix.mu).  Set
@@ -672,9 +792,9 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
   if (mode == B2K_MODE_U8) mode = B2K_MODE_AUTO;  // not integer pixels: the certified screens
   if (u8) mode = B2K_MODE_U8;
   if (mode == B2K_MODE_AUTO)
-    mode = (!ix.range_ok || k > kMaxK) ? B2K_MODE_EXACT
-           : (ix.d >= kTcMinD && ix.n >= kTcMinN) ? B2K_MODE_BF16
-                                         : B2K_MODE_FP32;
+    mode = (!ix.range_ok || k > kMaxK)    ? B2K_MODE_EXACT
+           : knn_on_tensor_cores(ix, m, k) ? B2K_MODE_BF16
+                                           : B2K_MODE_FP32;
   if (mode != B2K_MODE_EXACT && !u8 && (!ix.range_ok || k > kMaxK)) mode = B2K_MODE_EXACT;
   if (stats) {
     memset(stats, 0, sizeof(*stats));
@@ -1279,7 +1399,8 @@ static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int ex
                         bool counted = false, bool sort_rows = true) {
   StreamFree fr{st, {}};
   int rc;
-  int mode = (!admit_all && ix.d >= kTcMinD && ix.n >= kTcMinN) ? B2K_MODE_BF16 : B2K_MODE_FP32;
+  const int mode =
+      !admit_all && radius_on_tensor_cores(ix, R2) ? B2K_MODE_BF16 : B2K_MODE_FP32;
   if (mode == B2K_MODE_BF16 && (rc = ensure_bf16(ix))) return rc;
   const bool tc = mode == B2K_MODE_BF16;
   const int64_t bm = tc ? kTcBM : kSimtBM;

@@ -35,13 +35,17 @@ __host__ __device__ constexpr int operand_parts(int d) { return d <= 10 ? 3 : d 
 __host__ __device__ constexpr int operand_cols(int d) {
   return operand_parts(d) == 3 ? 6 * d : operand_parts(d) == 2 ? 3 * d : d;
 }
-// Narrowest rows AUTO and the radius search send to the tensor cores.  200,003
-// x 8 rows, 50,021 queries, k = 5: the call takes 2.60 ms (screen 2.05 ms), on
-// the CUDA cores 17.54 ms (screen 17.03 ms).  Rows of one or two features stay
-// there: at 10^6 rows a plane holds more rows inside the accumulation error
-// (16 ulp of ||x||^2 an addition) than the lists take.
+// Narrowest rows AUTO and the radius search may send to the tensor cores.
+// 200,003 x 8 rows, 50,021 queries, k = 5: the call takes 2.27 ms (screen 1.93),
+// on the CUDA cores 17.4 ms (screen 17.0).  Under 16 features the index's sample
+// (NarrowProfile) decides; rows of one or two features stay on the CUDA cores: at
+// 10^6 rows a plane holds more rows inside the accumulation error (16 ulp of
+// ||x||^2 an addition) than the lists take.
 constexpr int kTcMinD = 3;
+constexpr int kTcAlwaysD = 16;  // from here on whatever the data
 constexpr int64_t kTcMinN = 2048;
+constexpr int kProfileSamples = 64;
+constexpr int kProfileBins = 128;   // a quarter octave each, up to 4 max ||x - c||^2
 constexpr int kStatsLen = 12;  // floats of Index::stats_dev (prep.cu)
 constexpr int kSimtBM = 128; // query rows per CUDA-core tile
 constexpr int kSimtBN = 64;  // reference rows per CUDA-core tile
@@ -70,6 +74,26 @@ struct OperandStats {
   float part[3] = {0, 0, 0};  // ||hi||, ||mid||, ||lo|| (one part: ||x^||, 0, 0)
 };
 
+// How densely the rows of a narrow index lie: squared distances of
+// kProfileSamples rows to `rows` others spread over the index, as a histogram a
+// sample (prep.cu).
+//
+// The tensor-core screen certifies a value to within E, which grows with the
+// index's largest norm (its accumulation error is relative to ||x||^2, 768 times
+// the fp32 screen's at 8 features): one far row, a sentinel or an unscaled column
+// can put most of the index into the band of every query.  The rows are then
+// listed in vain and searched again by the fp32 screen.  200,003 N(0, 1) rows of
+// 8 features, 50,021 queries, k = 5, one row moved to distance r, tensor cores /
+// fp32 screen: r = 60 (85 rows in the median band) 3.3 / 17.4 ms, r = 100 (613,
+// 27% of the queries uncertified) 10.9 / 17.4, r = 150 (5,589) 68 / 17.4,
+// r = 300 (129,927) 64 / 17.5.
+struct NarrowProfile {
+  int rows = 0;               // 0: no sample taken
+  int base = 0;               // float bits >> 21 of the first bin
+  float rms = 0;              // median ||x - c|| of the samples
+  std::vector<int> cum;       // [samples][bins + 1] rows below each bin's lower edge
+};
+
 // Device-resident index (one per fitted estimator).
 struct Index {
   int device = 0;
@@ -84,6 +108,7 @@ struct Index {
   float* stats_dev = nullptr;  // [kStatsLen]: see prep kernels
   float xn_max = 0, nx_max = 0;  // max ||fp32 operand||, max ||x - center||^2
   float ex32_max = 0;            // max ||(x - center) - fp32 operand||
+  NarrowProfile profile;         // 3 <= d < 16
   bool range_ok = false;         // all |x| in {0} U [2^-60, 2^50]
   // bf16 copy for the tcgen05 screen (lazy)
   bool bf16_ready = false;
@@ -134,6 +159,11 @@ struct Index {
 
 // ------------------------------------------------------------ prep kernels
 void launch_prep_index(Index* ix, cudaStream_t st);
+// After launch_prep_index: the histograms of NarrowProfile (hist [samples][bins],
+// zeroed by the caller) and the samples' ||x - c||^2, of rows <= n others each
+int profile_rows(int64_t n);
+int profile_base(float nx_max);
+void launch_narrow_profile(const Index* ix, int rows, int* hist, double* norms, cudaStream_t st);
 // flag |= 1 when some value is NaN or infinite
 void launch_nonfinite_check(const float* v, int64_t count, int* flag, cudaStream_t st);
 // bf16 operand rows [n_pad, dp] (n_pad = n rounded up to 256) into Xh, row i

@@ -33,6 +33,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <cstring>
 
 #include "common.cuh"
 #include "internal.cuh"
@@ -113,6 +114,46 @@ __global__ void prep_index_kernel(const float* __restrict__ X, int64_t n, int d,
     atomic_max_pos(stats + 5, __double2float_ru(sqrt(ee) * (1.0 + 1e-15) + 0x1p-50 * sqrt(yy)));
     if (!ok) atomicAdd(reinterpret_cast<int*>(stats + 2), 1);
   }
+}
+
+__host__ __device__ inline int profile_base_of(uint32_t nx_bits_x4) {
+  return (int)(nx_bits_x4 >> 21) - (kProfileBins - 1);
+}
+
+// One sample a blockIdx.x, a slice of the other rows a blockIdx.y: direct squared
+// distances into the sample's histogram.  A few microseconds once an index (at
+// most 64 x 65,536 pairs of under 16 features), bound by the scattered row loads.
+constexpr int kProfileThreads = 256;
+__global__ void __launch_bounds__(kProfileThreads)
+    narrow_profile_kernel(const float* __restrict__ X, int64_t n, int d, int rows,
+                          const double* __restrict__ nx64, const float* __restrict__ stats,
+                          int* __restrict__ hist, double* __restrict__ norms) {
+  __shared__ int h[kProfileBins];
+  for (int i = threadIdx.x; i < kProfileBins; i += kProfileThreads) h[i] = 0;
+  __syncthreads();
+  const int s = blockIdx.x;
+  const int64_t own = (int64_t)s * n / kProfileSamples;
+  const int base = profile_base_of(__float_as_uint(4.0f * stats[1]));
+  float q[kTcAlwaysD - 1];
+#pragma unroll
+  for (int c = 0; c < kTcAlwaysD - 1; ++c) q[c] = c < d ? X[own * d + c] : 0.0f;
+  for (int i = blockIdx.y * kProfileThreads + threadIdx.x; i < rows;
+       i += gridDim.y * kProfileThreads) {
+    const int64_t row = (int64_t)i * n / rows;
+    if (row == own) continue;
+    float S = 0.0f;
+#pragma unroll
+    for (int c = 0; c < kTcAlwaysD - 1; ++c) {
+      const float e = c < d ? q[c] - X[row * d + c] : 0.0f;
+      S = fmaf(e, e, S);
+    }
+    const int b = (int)((__float_as_uint(S) & 0x7fffffffu) >> 21) - base;
+    atomicAdd(h + min(max(b, 0), kProfileBins - 1), 1);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kProfileBins; i += kProfileThreads)
+    if (h[i]) atomicAdd(hist + s * kProfileBins + i, h[i]);
+  if (blockIdx.y == 0 && threadIdx.x == 0) norms[s] = nx64[own];
 }
 
 // The bf16 parts of a centred fp32 value (the differences are exact in fp32).
@@ -458,6 +499,22 @@ void launch_prep_index(Index* ix, cudaStream_t st) {
   const int warps = 8;
   prep_index_kernel<<<(unsigned)((ix->n + warps - 1) / warps), warps * 32, 0, st>>>(
       ix->X, ix->n, ix->d, ix->center, ix->nx32, ix->nx64, ix->stats_dev);
+}
+
+int profile_rows(int64_t n) {
+  return (int)std::min<int64_t>(n, std::max<int64_t>(8192, std::min<int64_t>(n / 16, 65536)));
+}
+
+int profile_base(float nx_max) {
+  const float v = 4.0f * nx_max;
+  uint32_t bits;
+  memcpy(&bits, &v, sizeof(bits));
+  return profile_base_of(bits);
+}
+
+void launch_narrow_profile(const Index* ix, int rows, int* hist, double* norms, cudaStream_t st) {
+  narrow_profile_kernel<<<dim3(kProfileSamples, 8), kProfileThreads, 0, st>>>(
+      ix->X, ix->n, ix->d, rows, ix->nx64, ix->stats_dev, hist, norms);
 }
 
 void launch_prep_index_bf16(const Index* ix, uint16_t* Xh, cudaStream_t st, const int* rows) {

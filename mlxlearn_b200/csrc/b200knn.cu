@@ -401,16 +401,21 @@ static bool knn_on_tensor_cores(const Index& ix, int64_t m, int k) {
   return wide * 4 <= kProfileSamples;
 }
 
-// Whether the radius search sends its queries to the tensor cores: as
+// Whether the radius search sends a block of m queries to the tensor cores: as
 // above, by the rows in (R2, R2 + 2E] a query.  Every one is a candidate (12 bytes
 // of scratch and an exact test), so they are kept below 1,024, or below the
 // answer's own size: 200,003 x 8, 20,000 queries, 90 neighbours: 421 candidates 1.4
 // / 13.1 ms, 2,082 2.0, 38,007 6.9 ms and 9 GB, where the fp32 screen has 93.
-static bool radius_on_tensor_cores(const Index& ix, double R2) {
+// Small calls (pairs with the queries padded to a tile) are launches and host
+// reads, of which the list form has more than the fp32 screen's counted form:
+// 10,000 x 8, 500 queries: 232 / 167 us; 20,000 x 13, 500: 284 / 207; 50,000 x 8,
+// 500 (2.5e7 pairs): 273 / 247; 10,000 x 8, 4,000 (4e7): 229 / 310; 100,000 x 13,
+// 500: 328 / 359; 200,000 x 8, 1 (2.6e7): 263 / 367.
+static bool radius_on_tensor_cores(const Index& ix, int64_t m, double R2) {
   if (ix.d < kTcMinD || ix.n < kTcMinN) return false;
   if (ix.d >= kTcAlwaysD) return true;
   const NarrowProfile& p = ix.profile;
-  if (!p.rows) return false;
+  if (!p.rows || std::max<int64_t>(m, kTcBM) * ix.n < ((int64_t)3 << 23)) return false;
   const double band = 2.0 * profile_error(ix);
   double inside = 0, wide = 0;
   for (int s = 0; s < kProfileSamples; ++s) {
@@ -1400,7 +1405,7 @@ static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int ex
   StreamFree fr{st, {}};
   int rc;
   const int mode =
-      !admit_all && radius_on_tensor_cores(ix, R2) ? B2K_MODE_BF16 : B2K_MODE_FP32;
+      !admit_all && radius_on_tensor_cores(ix, m, R2) ? B2K_MODE_BF16 : B2K_MODE_FP32;
   if (mode == B2K_MODE_BF16 && (rc = ensure_bf16(ix))) return rc;
   const bool tc = mode == B2K_MODE_BF16;
   const int64_t bm = tc ? kTcBM : kSimtBM;

@@ -53,7 +53,7 @@ def test_equal_rows():
 # screen has no such wait and answers.  500 x 10,000 rows: a small call.
 @pytest.mark.parametrize("n,m,kind,tensor_cores", [
     (40_000, 1000, "normal", True), (40_000, 1000, "far", False),
-    (100_000, 300, "column", False)])
+    (100_000, 300, "column", False), (20_000, 500, "normal", False)])
 @pytest.mark.parametrize("d", [3, 8, 13])
 def test_radius_route(monkeypatch, n, m, kind, tensor_cores, d):
     X = _rows(n, d, kind)

@@ -863,11 +863,14 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
     // Register trackers (call with the pass / without): 8,192 x 64, 6,000 queries,
     // k = 5: 231 / 198 us; 120,000 x 15, 6,000: 426 / 393; 30,000 x 64, 20,000: 535
     // / 525 and 50,000: 974 / 1,040; 120,000 x 64, 20,000: 966 / 1,057; 500,000 x 15,
-    // 20,000, k = 15: 3,576 / 3,726.  A lazy tracker needs some threshold always.
+    // 20,000, k = 15: 3,576 / 3,726.  A lazy tracker needs some threshold always
+    // (as its pass keeps k values a row: with eight epilogue warps, B2K_TC_EW=8, its
+    // two column groups hold 32, and larger k take the spread pass below.)
+    const int seed_k = lazy ? 16 : k, seed_groups = tc ? tc_column_groups(seed_k) : 0;
     const bool seed = tc && grouped && ix.group_start && n_tiles >= 2 * kSeedTiles &&
                       seed_enabled() &&
-                      (lazy || (m_tiles >= sms && m_tiles * n_tiles >= 256 * (int64_t)sms));
-    const int seed_k = lazy ? 16 : k, seed_groups = tc ? tc_column_groups(seed_k) : 0;
+                      (lazy ? seed_groups * seed_k >= k
+                            : m_tiles >= sms && m_tiles * n_tiles >= 256 * (int64_t)sms);
     // Lazy lists without grouped queries (m < 2048 or few rows) are seeded from
     // windows spread over the rows: an eighth of the tiles, 4 to 64 (128 where the
     // units would otherwise leave SMs idle), in as many windows as keep two units
@@ -992,7 +995,7 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
                             cudaGetErrorString((cudaError_t)lr));
         if (spread)
           launch_seed_kth_spread(seed_kth, spread_S * seed_groups, m, m_pad, k, shared_kth, st);
-        else if (lazy && seed_groups * seed_k >= k)
+        else if (lazy)
           launch_seed_kth(seed_kth, seed_groups, seed_k, m, m_pad, k, shared_kth, st);
         if (stats) cudaEventRecord(ev[4], st);
         seeded = true;

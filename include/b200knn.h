@@ -113,9 +113,11 @@ B2K_API int b2k_index_download(const b2k_index *index, float *X);
 B2K_API const float *b2k_index_device_data(const b2k_index *index);
 
 /* Copy `bytes` of host memory to device memory on `stream` (of the current
- * device).  Pageable memory is staged through page-locked slots by a few host
- * threads while an index lives; the source may be reused on return.  No
- * counterpart in the reference (MLX arrays share memory with the host). */
+ * device).  The source may be reused on return: pageable memory has been staged
+ * (large arrays through page-locked slots by a few host threads while an index
+ * lives), for other memory (page-locked, managed) the call waits for the copy,
+ * unless the stream is being captured.  No counterpart in the reference (MLX
+ * arrays share memory with the host). */
 B2K_API int b2k_upload(void *d_dst, const void *src, int64_t bytes, void *stream);
 
 /* -------------------------------------------------------------------- kNN */

@@ -450,9 +450,11 @@ int knn_backward(const float* Q, int64_t m, const float* X, int64_t n, int d, in
 size_t knn_backward_workspace_ints(int64_t m, int64_t n, int k);
 
 // ---------------------------------------------------------- uploads (upload.cu)
-// Host to device copy on `st` of the current device; pageable sources go through
-// pinned staging while some index holds it.  The source may be reused on return.
-cudaError_t upload_host(void* dst, const void* src, size_t bytes, cudaStream_t st);
+// Host to device copy on `st` of the current device; large pageable sources go
+// through pinned staging while some index holds it.  A pageable source may be
+// reused on return, any other once `st` has passed the copy (*pageable tells).
+cudaError_t upload_host(void* dst, const void* src, size_t bytes, cudaStream_t st,
+                        bool* pageable = nullptr);
 void staging_acquire(int device);
 void staging_release(int device);
 

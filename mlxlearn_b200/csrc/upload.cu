@@ -4,8 +4,9 @@
 // queries (10,000 x 784) took 1.6 to 2.9 ms, two to four times the search behind
 // it.  Here up to four threads (the caller among them) copy 1 MB chunks into
 // pinned slots, two slots a thread, and enqueue each chunk's DMA as soon as it is
-// staged, so staging and DMA overlap: 31 MB in about 1 ms.  The copies of one call are
-// enqueued on the caller's stream; when it returns the source may be reused.
+// staged, so staging and DMA overlap: 31 MB in about 1 ms.  The copies of one call
+// are enqueued on the caller's stream; when it returns the pageable source may be
+// reused.
 //
 // The slots (8 MB a device) live as long as some index does.  One upload uses
 // them at a time; a concurrent one, a small one, or one whose source is already
@@ -85,17 +86,22 @@ void staging_release(int device) {
   s.buf = nullptr;
 }
 
-cudaError_t upload_host(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+cudaError_t upload_host(void* dst, const void* src, size_t bytes, cudaStream_t st,
+                        bool* pageable) {
   auto plain = [&] { return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st); };
-  if (bytes < kMinBytes) return plain();
+  // (a small internal copy is followed by a wait of its caller: no need to ask)
+  if (pageable) *pageable = false;
+  if (bytes < kMinBytes && !pageable) return plain();
   cudaPointerAttributes attr;
   if (cudaPointerGetAttributes(&attr, src) != cudaSuccess) {
     cudaGetLastError();
     return plain();
   }
+  const bool registered = attr.type != cudaMemoryTypeUnregistered;
+  if (pageable) *pageable = !registered;
+  if (bytes < kMinBytes || registered) return plain();
   int device = 0;
-  if (attr.type != cudaMemoryTypeUnregistered || cudaGetDevice(&device) != cudaSuccess ||
-      device < 0 || device >= kMaxDevices)
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices)
     return plain();
   Staging& s = staging(device);
   std::unique_lock<std::mutex> lock(s.mu, std::try_to_lock);
@@ -143,8 +149,13 @@ extern "C" B2K_API int b2k_upload(void* d_dst, const void* src, int64_t bytes, v
   if (bytes < 0) return report_error(B2K_EINVAL, "negative byte count");
   if (bytes == 0) return B2K_OK;
   if (!d_dst || !src) return report_error(B2K_EINVAL, "pointers must not be NULL");
-  const cudaError_t e =
-      upload_host(d_dst, src, (size_t)bytes, static_cast<cudaStream_t>(stream));
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  bool pageable = false;
+  cudaError_t e = upload_host(d_dst, src, (size_t)bytes, st, &pageable);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (e == cudaSuccess && !pageable) e = cudaStreamIsCapturing(st, &capture);
+  if (e == cudaSuccess && !pageable && capture == cudaStreamCaptureStatusNone)
+    e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return report_error(B2K_ECUDA, cudaGetErrorString(e));
   return B2K_OK;
 }

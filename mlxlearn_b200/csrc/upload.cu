@@ -99,7 +99,8 @@ cudaError_t upload_host(void* dst, const void* src, size_t bytes, cudaStream_t s
   }
   const bool registered = attr.type != cudaMemoryTypeUnregistered;
   if (pageable) *pageable = !registered;
-  if (bytes < kMinBytes || registered) return plain();
+  // (the per-thread default stream is another stream in each helper thread)
+  if (bytes < kMinBytes || registered || st == cudaStreamPerThread) return plain();
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices)
     return plain();

@@ -1,9 +1,11 @@
 """What b2k_upload promises: the source may be reused on return whatever memory it
-is, and the copy is ordered on the caller's stream."""
+is, and the copy is ordered on the caller's stream, the per-thread one included."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
+
+PER_THREAD = 2  # cudaStreamPerThread
 
 
 @pytest.fixture
@@ -19,7 +21,7 @@ def index():
 # below and above the size from which pageable memory is staged (16 MB)
 @pytest.mark.parametrize("nbytes", [1000, 3 * 2**20, 33 * 2**20 + 5])
 @pytest.mark.parametrize("memory", ["pageable", "pinned"])
-@pytest.mark.parametrize("stream", ["own", "legacy"])
+@pytest.mark.parametrize("stream", ["own", "per_thread", "legacy"])
 def test_source_is_free_and_stream_order_holds(index, nbytes, memory, stream):
     import torch
 
@@ -30,7 +32,8 @@ def test_source_is_free_and_stream_order_holds(index, nbytes, memory, stream):
     want = src.copy()
     dst = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
     torch.cuda.synchronize()
-    s = {"own": torch.cuda.Stream(), "legacy": torch.cuda.default_stream()}[stream]
+    s = {"own": torch.cuda.Stream(), "per_thread": torch.cuda.ExternalStream(PER_THREAD),
+         "legacy": torch.cuda.default_stream()}[stream]
     with torch.cuda.stream(s):
         torch.cuda._sleep(40_000_000)  # about 20 ms: the copy waits behind it
         dst.zero_()

@@ -189,10 +189,12 @@ static int dalloc(T** p, size_t count, cudaStream_t st) {
   *p = nullptr;
   if (count == 0) count = 1;
   cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(p), count * sizeof(T), st);
-  if (e != cudaSuccess)
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // (the next launch's check would report it again)
     return fail(e == cudaErrorMemoryAllocation ? B2K_ENOMEM : B2K_ECUDA,
                 "device allocation of %zu bytes failed: %s", count * sizeof(T),
                 cudaGetErrorString(e));
+  }
   return B2K_OK;
 }
 
@@ -211,9 +213,11 @@ static int ialloc(Index& ix, T** p, size_t count) {
   const bool pooled = bytes <= kPoolAlloc;
   void* v = nullptr;
   const cudaError_t e = pooled ? cudaMallocAsync(&v, bytes, ix.stream) : cudaMalloc(&v, bytes);
-  if (e != cudaSuccess)
+  if (e != cudaSuccess) {
+    cudaGetLastError();
     return fail(e == cudaErrorMemoryAllocation ? B2K_ENOMEM : B2K_ECUDA,
                 "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+  }
   ix.owned.emplace_back(v, pooled);
   *p = static_cast<T*>(v);
   return B2K_OK;
@@ -913,12 +917,6 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
     // the register trackers' lists hold 4 x kListCap entries per (split, query)
     // whatever the column groups (the lazy tracker's select is sized for kListCap)
     so.cap = (tc && !lazy) ? kListCap * 4 / tc_column_groups(k) : kListCap;
-    // (half of it in four lists a split where that would pass 32 GB, from about
-    // two million queries: two lists of kListCap hold as much, which is what
-    // eight epilogue warps, and the fp32 screen of rows under 16 features, take)
-    if ((lazy || (tc && ix.d < 16)) && tc_column_groups(k) == 4 &&
-        (size_t)S_lists * m_pad * kListCap * sizeof(int2) > ((size_t)32 << 30))
-      so.cap = kListCap / 2;
     so.m_pad = (int)m_pad;
     ws.reserve(&so.lists, (size_t)S_lists * m_pad * so.cap);
     ws.reserve(&so.counts, (size_t)S_lists * m_pad);
@@ -1102,6 +1100,71 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
   return B2K_OK;
 }
 
+// Queries of a call that one block answers.  The lazy tracker's four lists a split,
+// and those of rows under 16 features, take twice what the eight-warp form and the
+// fp32 screen take (16 KB against 8 a query and split), so these calls keep their
+// lists within 8 GB (B2K_KNN_LIST_MB) and answer larger batches block by block:
+// from about 160,000 queries at three splits, where a block fills the GPU many
+// times over.  Lists half as long would take the earlier memory too, but rows
+// whose certified band is wide then compact at every chunk: 1M x 128, k = 50,
+// 20,000 queries 12 -> 151 ms, 100,000: 33 -> 951.
+static int64_t knn_block_rows(const Index& ix, int64_t m, int k, int mode) {
+  const int base = mode & ~B2K_MODE_SQUARED;
+  if (base == B2K_MODE_FP32 || base == B2K_MODE_EXACT || k > kMaxK ||
+      !(tc_lazy_sink(k) || ix.d < kTcAlwaysD) || tc_column_groups(k) != 4)
+    return m;
+  const char* mb = getenv("B2K_KNN_LIST_MB");
+  const int64_t budget = std::max<int64_t>(1, mb ? atoll(mb) : 8192) << 20;
+  if (round_up(m, kTcBM) * kMaxSplits * 4 * kListCap * (int64_t)sizeof(int2) <= budget) return m;
+  const int64_t n_tiles = round_up(ix.n, kTcBN) / kTcBN;
+  for (int64_t blocks = 1;; blocks *= 2) {
+    const int64_t rows = round_up((m + blocks - 1) / blocks, kTcBM);
+    const int S = choose_splits(rows / kTcBM, n_tiles, num_sms(ix.device));
+    if (rows <= kTcBM || rows * S * 4 * kListCap * (int64_t)sizeof(int2) <= budget)
+      return blocks == 1 ? m : rows;
+  }
+}
+
+// The search of a public entry point: in blocks (knn_block_rows), and in smaller
+// ones where the device has no memory left for a block's scratch.  Answers do not
+// depend on the blocking.
+constexpr int64_t kLeastBlock = 8192;  // queries below which ENOMEM is returned
+static int knn_device(Index& ix, const float* dQ, int64_t m, int k, int exclude_self,
+                      int64_t q_offset, int mode, double* d_dist, int64_t* d_idx,
+                      cudaStream_t st, b2k_stats* stats) {
+  int64_t rows = knn_block_rows(ix, m, k, mode);
+  b2k_stats all{};
+  for (int64_t r0 = 0; r0 < m || m == 0;) {
+    const int64_t len = std::min(rows, m - r0);
+    b2k_stats one{};
+    const int rc = knn_device_impl(ix, dQ + r0 * ix.d, len, k, exclude_self, q_offset + r0, mode,
+                                   d_dist ? d_dist + r0 * k : nullptr, d_idx + r0 * k, st,
+                                   stats ? &one : nullptr);
+    if (rc == B2K_ENOMEM && len > kLeastBlock) {
+      rows = round_up((len + 1) / 2, kTcBM);
+      continue;
+    }
+    if (rc) return rc;
+    if (stats) {
+      all.mode_used = one.mode_used;
+      all.splits = one.splits;
+      all.candidates += one.candidates;
+      all.list_entries += one.list_entries;
+      all.fallback_rows += one.fallback_rows;
+      all.second_pass_rows += one.second_pass_rows;
+      all.exact_compares += one.exact_compares;
+      all.screen_ms += one.screen_ms;
+      all.total_ms += one.total_ms;
+      all.refined += one.refined;
+      all.seed_ms += one.seed_ms;
+      *stats = all;
+    }
+    r0 += len;
+    if (m == 0) break;
+  }
+  return B2K_OK;
+}
+
 static int validate_knn(const Index& ix, int64_t m, int32_t k, int32_t exclude_self,
                         int64_t q_offset, int32_t mode) {
   if (m < 0) return fail(B2K_EINVAL, "negative query count");
@@ -1128,7 +1191,7 @@ int check_knn_args(const Index& ix, int64_t m, int32_t k, int32_t exclude_self,
 Index* index_of(b2k_index* h) { return h ? &h->ix : nullptr; }
 int knn_device_run(Index& ix, const float* dQ, int64_t m, int k, int exclude_self,
                    int64_t q_offset, int mode, double* d_dist, int64_t* d_idx, cudaStream_t st) {
-  return knn_device_impl(ix, dQ, m, k, exclude_self, q_offset, mode, d_dist, d_idx, st, nullptr);
+  return knn_device(ix, dQ, m, k, exclude_self, q_offset, mode, d_dist, d_idx, st, nullptr);
 }
 int injected_fault() { return fault_mode(); }
 int index_prepare_bf16_stats(Index& ix, uint16_t* Xh, uint16_t* Xaug, uint16_t* ones,
@@ -1323,8 +1386,8 @@ int b2k_knn_device(b2k_index* h, const float* dQ, int64_t m, int32_t k, int32_t 
       overlaps(d_dist, (size_t)m * k * 8, dQ, (size_t)m * ix.d * 4) ||
       overlaps(d_idx, (size_t)m * k * 8, d_dist, (size_t)m * k * 8))
     return fail(B2K_EINVAL, "output buffers must not overlap inputs or each other");
-  return knn_device_impl(ix, dQ, m, k, exclude_self, q_offset, mode, d_dist, d_idx,
-                         (cudaStream_t)stream, stats);
+  return knn_device(ix, dQ, m, k, exclude_self, q_offset, mode, d_dist, d_idx,
+                    (cudaStream_t)stream, stats);
 }
 
 int b2k_knn(b2k_index* h, const float* Q, int64_t m, int32_t k, int32_t exclude_self,
@@ -1354,7 +1417,7 @@ int b2k_knn(b2k_index* h, const float* Q, int64_t m, int32_t k, int32_t exclude_
   }
   B2K_CUDA(upload_host(dQ, Q, (size_t)m * ix.d * sizeof(float), st));
   // finiteness is checked on the device inside the search (one pass over HBM)
-  rc = knn_device_impl(ix, dQ, m, k, exclude_self, q_offset, mode, dd, di, st, stats);
+  rc = knn_device(ix, dQ, m, k, exclude_self, q_offset, mode, dd, di, st, stats);
   if (rc) return rc;
   B2K_CUDA(cudaMemcpyAsync(idx, di, (size_t)m * k * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   if (dist)

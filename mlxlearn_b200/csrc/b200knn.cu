@@ -1446,14 +1446,16 @@ namespace b2k {
 // lists allows (B2K_RADIUS_LIST_MB), a multiple of 32 in [64, 1024], or 0 when
 // that budget holds fewer than 64 per list.  With 512 MB a few dense rows of
 // 100,003 x 24 (30,011 queries) and 200,000 x 32 (50,000) overflowed, and their
-// counted sub-call cost 0.25 of 2.57 ms and 0.2 of 4.55.
-static int radius_list_cap(int S_lists, int64_t m_pad) {
+// counted sub-call cost 0.25 of 2.57 ms and 0.2 of 4.55; `lean`, a call that found
+// no memory, is held to that budget.
+static int radius_list_cap(int S_lists, int64_t m_pad, bool lean) {
   if (const char* e = getenv("B2K_RADIUS_CAP")) {
     const long c = atol(e);
     return c <= 0 ? 0 : (int)std::min<long>(c, 1 << 20);
   }
   const char* mb = getenv("B2K_RADIUS_LIST_MB");
-  const int64_t budget = (int64_t)(mb ? atoll(mb) : 2048) << 20;
+  int64_t budget = (int64_t)(mb ? atoll(mb) : 2048) << 20;
+  if (lean) budget = std::min<int64_t>(budget, (int64_t)512 << 20);
   int64_t c = budget / ((int64_t)S_lists * m_pad * (int64_t)sizeof(int)) / 32 * 32;
   return c < 64 ? 0 : (int)std::min<int64_t>(c, 1024);
 }
@@ -1463,15 +1465,17 @@ static int radius_list_cap(int S_lists, int64_t m_pad) {
 // by a counted sub-call (count pass, then fill at scanned offsets) on those
 // rows alone, the form the CUDA-core screen always uses (`counted`).
 // qrows: the block row of each query for self-exclusion (sub-calls), or null.
+// lean: shorter lists, and narrow rows on the fp32 screen, whose candidates are few.
 // Stores device CSR pieces in `res` (which then owns them).
 static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int exclude_self,
                         int64_t q_offset, bool need_distance, bool sort_results, bool admit_all,
                         cudaStream_t st, b2k_radius_result* res, const int* qrows = nullptr,
-                        bool counted = false, bool sort_rows = true) {
+                        bool counted = false, bool sort_rows = true, bool lean = false) {
   StreamFree fr{st, {}};
   int rc;
-  const int mode =
-      !admit_all && radius_on_tensor_cores(ix, m, R2) ? B2K_MODE_BF16 : B2K_MODE_FP32;
+  const int mode = !admit_all && !(lean && ix.d < kTcAlwaysD) && radius_on_tensor_cores(ix, m, R2)
+                       ? B2K_MODE_BF16
+                       : B2K_MODE_FP32;
   if (mode == B2K_MODE_BF16 && (rc = ensure_bf16(ix))) return rc;
   const bool tc = mode == B2K_MODE_BF16;
   const int64_t bm = tc ? kTcBM : kSimtBM;
@@ -1481,7 +1485,7 @@ static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int ex
   const int S = choose_splits(m_pad / bm, n_tiles, tc ? sms : 2 * sms);
   // candidate lists per row: one per (split, column group of the screen)
   const int S_lists = S * (tc ? tc_radius_groups() : simt_column_groups(kSinkRadiusCount));
-  const int cap = (tc && !counted) ? radius_list_cap(S_lists, m_pad) : 0;
+  const int cap = (tc && !counted) ? radius_list_cap(S_lists, m_pad, lean) : 0;
 
   // the block's state, zeroed and read back as one; counters: [0] exact tests,
   // [2] overflowed rows, [3] candidates, [4] members
@@ -1555,7 +1559,7 @@ static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int ex
     return fail(B2K_ETIMEOUT, "a bounded device wait gave up (code %d)", hstatus[0]);
   if ((hstatus[4] & 1) && !admit_all)
     return radius_block(ix, dQ, m, R2, exclude_self, q_offset, need_distance, sort_results, true,
-                        st, res, qrows, counted, sort_rows);
+                        st, res, qrows, counted, sort_rows, lean);
   // the candidates in one array at their scanned offsets, as training rows
   // (grouped operand rows are mapped); rows are re-sorted by index after the
   // compaction when their lists are out of index order (grouped rows, or
@@ -1620,13 +1624,15 @@ static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int ex
     sub = new b2k_radius_result();
     sub->device = ix.device;
     if ((rc = radius_block(ix, Qo, n_ovf, R2, exclude_self, q_offset, keep_dist, false, admit_all,
-                           st, sub, orow, true, false)))
+                           st, sub, orow, true, false, lean)))
       return rc;
     launch_radius_sub_counts(ovf, n_ovf, sub->indptr, ra.mcount, st);
   }
 
+  StreamFree out{st, {}};  // the result's arrays, until `res` owns them
   int64_t* indptr = nullptr;
   if ((rc = dalloc(&indptr, (size_t)m + 1, st))) return rc;
+  out.keep(indptr);
   launch_scan_rows(ra.mcount, m, indptr, scan_scratch, st);
   B2K_CUDA(cudaGetLastError());
   B2K_CUDA(cudaMemcpyAsync(counters + 4, indptr + m, sizeof(int64_t), cudaMemcpyDeviceToDevice,
@@ -1634,20 +1640,15 @@ static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int ex
   B2K_CUDA(cudaMemcpyAsync(&h, state, sizeof(h), cudaMemcpyDeviceToHost, st));
   B2K_CUDA(cudaStreamSynchronize(st));
   const int64_t nnz = (int64_t)h.counters[4];
-  if (hstatus[0] != DEV_OK) {  // the fill pass gave up (classify skipped its rows)
-    cudaFreeAsync(indptr, st);
+  if (hstatus[0] != DEV_OK)  // the fill pass gave up (classify skipped its rows)
     return fail(B2K_ETIMEOUT, "a bounded device wait gave up (code %d)", hstatus[0]);
-  }
   int64_t* indices = nullptr;
   double* dist = nullptr;
-  if ((rc = dalloc(&indices, (size_t)nnz, st))) {
-    cudaFreeAsync(indptr, st);
-    return rc;
-  }
-  if (keep_dist && (rc = dalloc(&dist, (size_t)nnz, st))) {
-    cudaFreeAsync(indptr, st);
-    cudaFreeAsync(indices, st);
-    return rc;
+  if ((rc = dalloc(&indices, (size_t)nnz, st))) return rc;
+  out.keep(indices);
+  if (keep_dist) {
+    if ((rc = dalloc(&dist, (size_t)nnz, st))) return rc;
+    out.keep(dist);
   }
   launch_compact(ra, indptr, indices, dist, st);
   if (sub)
@@ -1687,6 +1688,7 @@ static int radius_block(Index& ix, const float* dQ, int64_t m, double R2, int ex
     }
   }
   B2K_CUDA(cudaStreamSynchronize(st));
+  out.ptrs.clear();
   if (!need_distance && dist) {
     cudaFree(dist);
     dist = nullptr;
@@ -1748,9 +1750,13 @@ int b2k_radius(b2k_index* h, const float* Q, int64_t m, double radius, int32_t e
     return fail(B2K_ECUDA, "upload of the queries: %s", cudaGetErrorString(e));
   }
   // (NaN / inf queries are found by the block's query preparation)
-  rc = radius_block(ix, dQ, m, R2, exclude_self, q_offset, need_distance != 0,
-                    sort_results != 0 && sort_results != B2K_RADIUS_ANY_ORDER, !ix.range_ok, st,
-                    res, nullptr, false, sort_results != B2K_RADIUS_ANY_ORDER);
+  const bool ordered = sort_results != B2K_RADIUS_ANY_ORDER;
+  for (const bool lean : {false, true}) {
+    rc = radius_block(ix, dQ, m, R2, exclude_self, q_offset, need_distance != 0,
+                      ordered && sort_results != 0, !ix.range_ok, st, res, nullptr, false, ordered,
+                      lean);
+    if (rc != B2K_ENOMEM) break;
+  }
   cudaFreeAsync(dQ, st);
   cudaStreamSynchronize(st);
   if (rc) {

@@ -175,9 +175,9 @@ class RadiusCSR:
             # integer votes: their sum is the count, and the division rounds as
             # numpy's does
             out /= counts.clamp(min=1).unsqueeze(1)
-        host = _page_locked(out.numel(), np.float64)
-        torch.from_numpy(host).copy_(out.view(-1))
-        return host.reshape(out.shape), counts.cpu().numpy()
+        # (ordinary memory: a program keeps these arrays, and page-locked blocks
+        # would stay pinned with them)
+        return out.cpu().numpy(), counts.cpu().numpy()
 
     def votes(self, codes, n_classes: int, weighted: bool, proba: bool = False):
         """Per-row class votes (float64 ``[m, n_classes]``: weight 1, or 1/d

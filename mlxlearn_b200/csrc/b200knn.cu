@@ -372,7 +372,7 @@ static double profile_radius2(const NarrowProfile& p, int s, double rows) {
 // The certified error of the tensor-core screen for a query at the samples'
 // median distance from the centre (prep.cu derives it).
 static double profile_error(const Index& ix) {
-  const double g = (double)(round_up(ix.d, kTcBK) + kTcAug + 16) * 0x1p-20;
+  const double g = (double)(operand_dp(ix.d) + kTcAug + 16) * 0x1p-20;
   return 1.02 * g * (2.0 * ix.profile.rms * ix.xn_max + ix.nx_max);
 }
 
@@ -516,7 +516,7 @@ static int ensure_bf16(Index& ix) {
   std::lock_guard<std::mutex> lock(ix.mu);
   if (ix.bf16_ready) return B2K_OK;
   cudaStream_t st = ix.stream;
-  ix.dp = (int32_t)round_up(ix.d, kTcBK);
+  ix.dp = (int32_t)operand_dp(ix.d);
   ix.n_pad_tc = round_up(ix.n, kTcBN);
   int rc;
   if ((rc = ensure_row_groups(ix))) return rc;

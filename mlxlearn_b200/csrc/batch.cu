@@ -204,7 +204,7 @@ int build_fixed(b2k_batch* b, cudaStream_t st) {
   for (auto& p : b->probs) {
     if (!p.in_graph) continue;
     p.gi = gi++;
-    p.dp = (int)rup(p.ix->d, kTcBK);
+    p.dp = operand_dp(p.ix->d);
     p.KB = p.dp / kTcBK;
     p.n_tiles = (int)(rup(p.ix->n, kTcBN) / kTcBN);
     p.m_pad = (int)rup(p.m, kTcBM);

@@ -24,16 +24,26 @@ constexpr int kU8MaxD = 16384;  // ||x||^2 and -2<q, x> of u8 rows fit int32
 // Narrow rows leave most of a 64-column operand block empty, and the block
 // costs the same full or not (the epilogue bounds a 128 x 256 tile: multiplying
 // only the used columns was measured and was 2 to 4% slower).  So rows of at
-// most 21 features are split into bf16 parts (hi + mid, up to 10 features
-// hi + mid + lo) whose cross products fill the block: <q, x> then carries 16 or
-// 24 bits instead of 8, and the certified band shrinks with it.  With whole
-// bf16 operands the band of an 8-feature row (about 0.1 against a k-th squared
-// distance of 0.3 on 200,000 N(0, 1) rows) would hold most of a query's lists.
-__host__ __device__ constexpr int operand_parts(int d) { return d <= 10 ? 3 : d <= 21 ? 2 : 1; }
+// most 21 features are split into bf16 parts whose cross products fill the
+// block: hi + mid from 16 features on, so <q, x> carries 16 bits instead of 8,
+// and hi + mid + lo under 16, the 24 bits of the fp32 screen's operands.  With
+// whole bf16 operands the certified band of an 8-feature row (about 0.1 against a
+// k-th squared distance of 0.3 on 200,000 N(0, 1) rows) would hold most of a
+// query's lists.  11 to 15 features take a second block for the third part
+// (hi + mid fit one): 200,003 x 15, 50,021 queries, k = 5: 2.48 -> 2.90 ms; 1M x
+// 15, 20,000: 3.76 -> 4.77 (fp32 screen 34).
+constexpr int kTcAlwaysD = 16;  // narrower rows: fp32 precision, NarrowProfile's rule
+__host__ __device__ constexpr int operand_parts(int d) {
+  return d < kTcAlwaysD ? 3 : d <= 21 ? 2 : 1;
+}
 // operand columns in use: parts 2 = (h,h)(h,m)(m,h), parts 3 adds
 // (m,m)(h,l)(l,h), written (query part, row part)
 __host__ __device__ constexpr int operand_cols(int d) {
   return operand_parts(d) == 3 ? 6 * d : operand_parts(d) == 2 ? 3 * d : d;
+}
+// operand width, padded to whole blocks
+__host__ __device__ constexpr int operand_dp(int d) {
+  return (operand_cols(d) + kTcBK - 1) / kTcBK * kTcBK;
 }
 // Narrowest rows AUTO and the radius search may send to the tensor cores.
 // 200,003 x 8 rows, 50,021 queries, k = 5: the call takes 2.27 ms (screen 1.93),
@@ -42,7 +52,6 @@ __host__ __device__ constexpr int operand_cols(int d) {
 // 10^6 rows a plane holds more rows inside the accumulation error (16 ulp of
 // ||x||^2 an addition) than the lists take.
 constexpr int kTcMinD = 3;
-constexpr int kTcAlwaysD = 16;  // from here on whatever the data
 constexpr int64_t kTcMinN = 2048;
 constexpr int kProfileSamples = 64;
 constexpr int kProfileBins = 128;   // a quarter octave each, up to 4 max ||x - c||^2

@@ -520,7 +520,7 @@ void launch_narrow_profile(const Index* ix, int rows, int* hist, double* norms, 
 void launch_prep_index_bf16(const Index* ix, uint16_t* Xh, cudaStream_t st, const int* rows) {
   const int warps = 8;
   const int64_t n_pad = (ix->n + kTcBN - 1) / kTcBN * kTcBN;
-  const int dp = (ix->d + kTcBK - 1) / kTcBK * kTcBK;
+  const int dp = operand_dp(ix->d);
   const int64_t blocks = (n_pad + warps - 1) / warps;
   prep_index_bf16_kernel<<<(unsigned)blocks, warps * 32, 0, st>>>(
       ix->X, ix->n, ix->d, n_pad, dp, ix->center, rows, reinterpret_cast<__nv_bfloat16*>(Xh),
@@ -563,7 +563,7 @@ PrepProblem prep_problem(const Index* ix, const float* Q, int64_t m, int64_t m_p
   P.m = m;
   P.m_pad = m_pad;
   P.d = ix->d;
-  P.dp = tf32 ? (ix->d + kTcBKf - 1) / kTcBKf * kTcBKf : (ix->d + kTcBK - 1) / kTcBK * kTcBK;
+  P.dp = tf32 ? (ix->d + kTcBKf - 1) / kTcBKf * kTcBKf : operand_dp(ix->d);
   P.mode = mode;
   P.center = ix->center;
   P.parts = bf16 ? operand_parts(ix->d) : 1;

@@ -137,8 +137,9 @@ class KnnSegmentDistances(torch.autograd.Function):
         dist64, idx = _segments_forward(Qc, Xc, q_sizes, x_sizes, k, exclude_self)
         xo = _offsets(x_sizes)
         # global reference rows for the backward
-        starts, sizes = torch.as_tensor(np.stack([xo[:-1], np.asarray(q_sizes, np.int64)]),
-                                        device=Qc.device)
+        # (reference segments past the last query segment are not searched)
+        starts, sizes = torch.as_tensor(
+            np.stack([xo[:len(q_sizes)], np.asarray(q_sizes, np.int64)]), device=Qc.device)
         # (with its output size known, no read back of the sizes)
         gidx = idx + torch.repeat_interleave(starts, sizes,
                                              output_size=Qc.shape[0]).unsqueeze(1)

@@ -32,6 +32,8 @@ def _segments_forward(Qc, Xc, q_sizes, x_sizes, k, exclude_self):
     np.cumsum(np.asarray(x_sizes, dtype=np.int64), out=xo[1:])
     if qo[-1] != Qc.shape[0] or xo[-1] != Xc.shape[0]:
         raise ValueError("segment sizes must add up to the row counts")
+    if len(x_sizes) < len(q_sizes):
+        raise ValueError("every query segment needs a reference segment")
     rows, d = Qc.shape
     idx = torch.empty((rows, k), dtype=torch.int64, device=Qc.device)
     dist64 = torch.empty((rows, k), dtype=torch.float64, device=Qc.device)

@@ -1,7 +1,15 @@
-"""Segment lists of unequal length: reference segments may be left over."""
+"""Segment lists of unequal length: reference segments may be left over, query
+segments may not."""
 import numpy as np
 import pytest
 import torch
+
+
+def test_query_segment_without_reference_segment():
+    from mlxlearn_b200.autograd import _segments_forward
+
+    with pytest.raises(ValueError, match="reference segment"):
+        _segments_forward(torch.zeros(5, 3), torch.zeros(4, 3), (2, 3), (4,), 1, False)
 
 
 @pytest.mark.gpu

@@ -856,7 +856,7 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
     S = choose_splits(m_pad / bm, n_tiles, tc ? sms : 2 * sms);
     const bool lazy = tc && tc_lazy_sink(k);  // its screen leaves V_k to the lists
     // lists per query: one per (split, column group of the screen)
-    const int S_lists = S * (tc ? tc_column_groups(k) : simt_column_groups(kSinkKnn));
+    const int S_lists = S * (tc ? tc_column_groups() : simt_column_groups(kSinkKnn));
     // Group nearby queries (reorder.cu); results go back to the original rows.
     const bool grouped = !ext_perm && m >= 2048 && reorder_enabled();
     if (grouped && (rc = ensure_pivots(ix))) return rc;
@@ -870,7 +870,7 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
     // 20,000, k = 15: 3,576 / 3,726.  A lazy tracker needs some threshold always
     // (as its pass keeps k values a row: with eight epilogue warps, B2K_TC_EW=8, its
     // two column groups hold 32, and larger k take the spread pass below.)
-    const int seed_k = lazy ? 16 : k, seed_groups = tc ? tc_column_groups(seed_k) : 0;
+    const int seed_k = lazy ? 16 : k, seed_groups = tc ? tc_column_groups() : 0;
     const bool seed = tc && grouped && ix.group_start && n_tiles >= 2 * kSeedTiles &&
                       seed_enabled() &&
                       (lazy ? seed_groups * seed_k >= k
@@ -916,7 +916,7 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
     if (tf32) ws.reserve(&qp.At, (size_t)m_pad * ix.dpt);
     // the register trackers' lists hold 4 x kListCap entries per (split, query)
     // whatever the column groups (the lazy tracker's select is sized for kListCap)
-    so.cap = (tc && !lazy) ? kListCap * 4 / tc_column_groups(k) : kListCap;
+    so.cap = (tc && !lazy) ? kListCap * 4 / tc_column_groups() : kListCap;
     so.m_pad = (int)m_pad;
     ws.reserve(&so.lists, (size_t)S_lists * m_pad * so.cap);
     ws.reserve(&so.counts, (size_t)S_lists * m_pad);
@@ -1111,7 +1111,7 @@ static int knn_device_impl(Index& ix, const float* dQ, int64_t m, int k, int exc
 static int64_t knn_block_rows(const Index& ix, int64_t m, int k, int mode) {
   const int base = mode & ~B2K_MODE_SQUARED;
   if (base == B2K_MODE_FP32 || base == B2K_MODE_EXACT || k > kMaxK ||
-      !(tc_lazy_sink(k) || ix.d < kTcAlwaysD) || tc_column_groups(k) != 4)
+      !(tc_lazy_sink(k) || ix.d < kTcAlwaysD) || tc_column_groups() != 4)
     return m;
   const char* mb = getenv("B2K_KNN_LIST_MB");
   const int64_t budget = std::max<int64_t>(1, mb ? atoll(mb) : 8192) << 20;

@@ -9,9 +9,10 @@
 //   dX_r   = sum_{(i,j): idx(i,j) = r} c_ij (x_r - q_i)
 // dQ is a per-row reduction.  dX is a scatter-add made deterministic without
 // float atomics: the (i, j) pairs are bucketed by reference row with a
-// counting sort, each bucket is put in ascending flat order i*k + j, and every
-// bucket is summed by one warp in that order.  Results are bitwise identical
-// from run to run.
+// counting sort, each bucket is put in ascending flat order i*k + j and summed in
+// that order: by a thread up to eight features, by a warp above, and by a block
+// where more than kBigBucket queries picked the row.  Results are bitwise
+// identical from run to run.
 //
 // The reference has no differentiable kNN; this is the building block for
 // point-set losses such as a Chamfer term.

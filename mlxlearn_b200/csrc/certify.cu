@@ -2,10 +2,13 @@
 //
 // certify_kernel (one warp per query) turns the screen's candidate lists into
 // the final answer:
-//   1. V_k = k-th smallest screen value over all splits (bisection over the
-//      splits' k smallest values); threshold Tf = V_k + 2E (rounded up).
-//   2. Candidates = list entries with v <= Tf (tracker.cuh proves that no other
-//      row can be in the answer).
+//   1. V_k = k-th smallest screen value over all lists; threshold V_k + 2E
+//      (rounded up).  Lists without k-th values of their own, and many lists,
+//      are first cut to the entries within 2E of the row's shared word B >= V_k,
+//      and V_k is selected among those; otherwise from the lists' k smallest
+//      values (warp minima over up to 32 lists, a radix select over more).
+//   2. Candidates = list entries at or below the threshold (tracker.cuh proves
+//      that no other row can be in the answer).
 //   3. fp32 refinement with a certified relative bound, in two stages when
 //      the query's squared norm is known: first the k candidates with the
 //      smallest screen values, whose k-th smallest upper bound U0 then drops

@@ -257,7 +257,7 @@ int launch_screen_tc(Index* ix, const CUtensorMap* tmap_a, int64_t m, int64_t m_
 int launch_screen_tc_u8(Index* ix, const CUtensorMap* tmap_a, int64_t m, int64_t m_pad,
                         int exclude_self, int64_t q_offset, int S, const SinkArgs& sa,
                         int* status, cudaStream_t st, int* unit_counter);
-int tc_column_groups(int k);
+int tc_column_groups();
 int tc_u8_column_groups(int k);  // lists per (split, row) of the u8 screen
 int tc_radius_groups();  // candidate lists per (split, row) of the tcgen05 radius screens
 bool tc_lazy_sink(int k);  // the tcgen05 kNN screen's lazy tracker (no k-th output)

@@ -21,14 +21,15 @@
 //               accumulator: the thread issuing MMAs runs only about one MMA
 //               ahead of the tensor pipe, so a single issuer idles it while
 //               it waits for the next tile's operands and accumulator and
-//               while it commits.  One issuer behind a gate warp (which
-//               polled for it and cost two barrier hops a tile) took 2,130
-//               cycles a 128 x 256 x 144 tile, two issuers take 1,800 (1,152
-//               of MMA); 1,500 -> 1,450 at 64 columns, where the epilogue
-//               bounds the tile.  At 1M x 128 the clock falls with the busier
-//               pipe (the call is then bound by power), so the screen gains
-//               2%; 200,003 x 8: 2.01 -> 1.93 ms, 60,000 x 784 (one issuer,
-//               no gate): 1.06 -> 0.99 ms.
+//               while it commits.  1M x 128, 20,000 queries, ncu: one issuer
+//               behind a gate warp (which polled for it and cost two barrier
+//               hops a tile) 2,155 cycles a 128 x 256 x 144 tile over the
+//               whole launch (1,152 of MMA), two issuers 2,052; at 64
+//               columns, where the epilogue bounds the tile, 1,475 (640 of
+//               MMA).  At 100,000 queries the clock falls with the busier
+//               pipe (the call is then bound by power) and the gain is lost
+//               in the noise of a box; 200,003 x 8: 2.01 -> 1.93 ms, 60,000 x
+//               784 (one issuer, no gate): 1.06 -> 0.99 ms.
 //               Where the ring holds less than two tiles the first issuer
 //               issues all, each block as it lands.
 //   warps 2..   EW epilogue warps.  Warp w reads TMEM lane group w % 4 (the
@@ -48,8 +49,9 @@
 // per (split, column group, row).
 //
 // Operands are the centred coordinates rounded to bf16 (A = -2 bf16(q - c),
-// B = bf16(x - c); narrow rows in bf16 parts, operand_parts); the certified error bound of v is derived in prep.cu with
-// g = (dp + 32) 2^-20 for the tensor-core fp32 accumulation.
+// B = bf16(x - c); narrow rows in bf16 parts, operand_parts); the certified error
+// bound of v is derived in prep.cu with g = (dp + 32) 2^-20 for the tensor-core
+// fp32 accumulation.
 //
 // The TF32 instantiation is the plain (full-width) form on the tensor cores:
 // kind::tf32 MMAs (M=128, N=256, K=8) over operands rounded to tf32.  In bytes
@@ -694,23 +696,24 @@ int launch_tc_variant(const TcMapSet<BATCH ? kBatchGroups : 1>& maps, const TcPa
 
 }  // namespace
 
-// Column groups (epilogue warps per TMEM lane group) of the kNN screen for k:
-// each group keeps its own candidate lists.
+// Column groups (epilogue warps per TMEM lane group) of the kNN screen: each
+// group keeps its own candidate lists.
 // Epilogue warps of the single-problem kNN screen: four per TMEM lane group,
 // which shortens each warp's per-tile chain and cuts the issuers' waits for a
 // free accumulator (B2K_TC_EW=8 selects two).  The lazy tracker (k > 16) gains
 // twice: its lists hold kListCap entries each, so four a split also keep rows
-// whose certified band is wide from compacting at every chunk (1M x 128, 20,000
-// queries, k = 50: 216 ms with eight warps, 6.4 with sixteen; 200,000 x 64,
-// k = 32: 3.37 and 2.16).
-static int tc_knn_ew(int k) {
+// whose certified band is wide from compacting at every chunk.  Screen, seeding
+// included, with eight / sixteen warps: 1M x 128 mixture, 20,000 queries, k = 50:
+// 175 / 6.4 ms (sixteen warps with lists half as long: 122); 200,000 x 64, 50,000
+// queries, k = 32: 8.0 / 4.9; 60,013 x 100 against itself, k = 50: 3.8 / 1.7.
+static int tc_knn_ew() {
   static const int ew = [] {
     const char* e = getenv("B2K_TC_EW");
     return (e && atoi(e) == 8) ? 8 : 16;
   }();
   return ew;
 }
-int tc_column_groups(int k) { return tc_knn_ew(k) / 4; }
+int tc_column_groups() { return tc_knn_ew() / 4; }
 // Radius screens: four epilogue warps per TMEM lane group, one list per
 // (split, column group, row).
 constexpr int kRadiusEW = 16;
@@ -758,7 +761,7 @@ int launch_screen_tc(Index* ix, const CUtensorMap* tmap_a, int64_t m, int64_t m_
 #define B2K_TC_LAUNCH_TF32(SINK, EW)                                                 \
   (a_stream ? launch_tc_variant<SINK, true, EW, false, kKindTf32>(maps, p, KB, grid, st) \
             : launch_tc_variant<SINK, false, EW, false, kKindTf32>(maps, p, KB, grid, st))
-    if (tc_knn_ew(sa.k) == 16) {
+    if (tc_knn_ew() == 16) {
       if (sa.k <= 8) return B2K_TC_LAUNCH_TF32(KnnSink<8>, 16);
       if (sa.k <= 12) return B2K_TC_LAUNCH_TF32(KnnSink<12>, 16);
       if (!tc_lazy_sink(sa.k)) return B2K_TC_LAUNCH_TF32(KnnSink<16>, 16);
@@ -776,7 +779,7 @@ int launch_screen_tc(Index* ix, const CUtensorMap* tmap_a, int64_t m, int64_t m_
   if (sink_kind == kSinkRadiusCount) return B2K_TC_LAUNCH(RadiusCountSink, kRadiusEW);
   if (sink_kind == kSinkRadiusFill) return B2K_TC_LAUNCH(RadiusFillSink, kRadiusEW);
   if (sink_kind == kSinkRadiusList) return B2K_TC_LAUNCH(RadiusListSink, kRadiusEW);
-  if (tc_knn_ew(sa.k) == 16) {
+  if (tc_knn_ew() == 16) {
     if (sa.k <= 8) return B2K_TC_LAUNCH(KnnSink<8>, 16);
     if (sa.k <= 12) return B2K_TC_LAUNCH(KnnSink<12>, 16);
     if (!tc_lazy_sink(sa.k)) return B2K_TC_LAUNCH(KnnSink<16>, 16);
@@ -826,7 +829,7 @@ int launch_screen_tc_u8(Index* ix, const CUtensorMap* tmap_a, int64_t m, int64_t
 // 8 warps (two TMEM loads in flight each) for k = 9..16
 int tc_u8_column_groups(int k) { return k <= 8 ? 4 : 2; }
 
-// Batched launches: kNN sinks only, with 4 or 8 epilogue warps.  Heap width
+// Batched launches: kNN sinks only, with 4, 8 or 16 epilogue warps.  Heap width
 // class 64 stands for the lazy tracker (every k > 16).
 #define B2K_TC_BATCH_DISPATCH(CALL)                                         \
   switch (kmax * 32 + ew) {                                                 \

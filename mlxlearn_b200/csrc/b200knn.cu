@@ -388,12 +388,14 @@ static double profile_error(const Index& ix) {
 //   0.187 / 0.369.  20,000 x 5, 100 queries, k = 5: 110 0.137 / 0.098.
 // The predicted share agrees with the measured one to a few percent over normal,
 // uniform, heavy-tailed and clustered rows and one far row or column.
-static bool knn_on_tensor_cores(const Index& ix, int64_t m, int k) {
+static bool knn_on_tensor_cores(Index& ix, int64_t m, int k) {
   if (ix.d < kTcMinD || ix.n < kTcMinN) return false;
   if (ix.d >= kTcAlwaysD) return true;
   const NarrowProfile& p = ix.profile;
   if (!p.rows) return false;
   const bool small = m * ix.n < ((int64_t)1 << 28);
+  std::atomic<signed char>& known = ix.profile.knn[small ? 0 : 1][k];
+  if (const signed char said = known.load(std::memory_order_relaxed)) return said > 0;
   const double limit = small ? 2.0 * k + 32.0 : 1024.0;
   const double scale = (double)ix.n / p.rows;
   const double kth = std::max(1.0, k / scale), band = 2.0 * profile_error(ix);
@@ -402,7 +404,9 @@ static bool knn_on_tensor_cores(const Index& ix, int64_t m, int k) {
     const double t = profile_radius2(p, s, kth);
     if ((profile_within(p, s, t + band) - kth) * scale + k > limit) ++wide;
   }
-  return wide * 4 <= kProfileSamples;
+  const bool fits = wide * 4 <= kProfileSamples;
+  known.store(fits ? 1 : -1, std::memory_order_relaxed);
+  return fits;
 }
 
 // Whether the radius search sends a block of m queries to the tensor cores: as
